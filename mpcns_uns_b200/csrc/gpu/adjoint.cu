@@ -1864,6 +1864,7 @@ int mhd_gpu_fn_create(MhdState *st, const MhdFnParams *p, const double *eta, con
         fn->X0P.alloc(nf);
         copy_d(fn->X0U.p, st->U0.p, 5 * fn->nsp * nc, s);
         copy_d(fn->X0P.p, st->phi0.p, nf, s);
+        st->grad.alloc(15 * nc * st->group); // the recorded stages and the tangent run keep the gradients
         st->mres.alloc(ne);
         fn->active.alloc(nf);
         fn->rslot.alloc(4 * nc);

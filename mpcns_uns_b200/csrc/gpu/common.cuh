@@ -128,6 +128,31 @@ __device__ __forceinline__ void st3(double *a, int64_t i, V3 v)
     a[3 * i + 2] = v.z;
 }
 
+// 32 bytes in one access (sm_100's 256-bit global loads and stores); p 32-byte aligned
+struct alignas(32) D4
+{
+    double x, y, z, w;
+};
+__device__ __forceinline__ D4 ld_d4(const double *p)
+{
+    D4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_d4(double *p, double x, double y, double z, double w)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(w) : "memory");
+}
+
+// asynchronous 8-byte copies from global to shared memory
+__device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
+{
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
 // A field of `ncomp` values per entity: value(i, m) = p[i * si + m * sm].  The reference's
 // layout (AoS) is si = ncomp, sm = 1; the species-major state of the fused step is si = 1,
 // sm = n.
@@ -153,10 +178,11 @@ struct MeshView
     int32_t max_valence; // largest number of faces at an edge
     int32_t max_edge_cells; // largest number of cells at an edge (ec rows)
     int32_t tri_faces;      // 1 when every face is a triangle
-    int32_t faces_per_cell; // 4 when every cell is a tetrahedron (c2f row k of cell c at 4c), else 0
-    const double *st_dx; // face_center - cell_center per c2f entry (3 each)
-    // tetrahedral meshes only: the stencil as structure of arrays over cells, slot j of cell c at
-    // [j*nc + c] (coalesced warp loads): neighbour code, c2f sign, w*d (3 per slot), dx (3 per slot), inverse (6)
+    int32_t faces_per_cell; // 4 when every cell is a tetrahedron (c2f row k of cell c at 4c), 6 when every cell has six faces, else 0
+    const double *st_dx; // face_center - cell_center per c2f entry (3 each); null with faces_per_cell
+    // faces_per_cell > 0 only: the stencil as structure of arrays over cells, slot j of cell c at
+    // [j*nc + c] (coalesced warp loads): neighbour code, c2f sign, w*d (3 per slot), dx (3 per slot), inverse (6); the
+    // rows of t_wd, t_dx and t_inv follow one another in one array
     const int32_t *t_nb;
     const int8_t *t_sg;
     const double *t_wd, *t_dx, *t_inv;
@@ -169,6 +195,13 @@ struct MeshView
     const int32_t *f2c_ptr, *f2c_idx;
     const int8_t *f2c_sgn;
     const int32_t *face_L, *face_R; // cell with c2f sign +1 / -1 (canonical normal from L to R), -1 if none
+    // per face, read as one 32-byte and one 16-byte record: the unit normal (1/|A|) A_f and |A|; and the face's
+    // place in the fluid flux: (c2f entry of the L state, of the R state, FaceFlux | face_kind << 4, 0)
+    const double *fna;
+    const int4 *frec;
+    // per cell, entry (i, j) at [(3i + j)*nc + c]: the inverse of the cell-field fit's normal matrix
+    // sum |A| n n^T (zero where the fit is skipped)
+    const double *cinv;
     const int32_t *cfa_idx;         // c2f rows re-ordered by ascending face id (the reference's scatter order)
     const int8_t *cfa_sgn;
     const int8_t *material, *face_kind, *edge_mode;
@@ -179,14 +212,18 @@ struct MeshView
     const double *ec_weight, *ef_weight, *star1, *star2;
     // least-squares stencil of mhd::Stencil (per c2f entry / per cell)
     const int32_t *st_nb;    // neighbour cell, -(f+1) for a virtual boundary neighbour, INT32_MIN for a skipped face
-    const double *st_wd;     // w * d (3 per c2f entry)
-    const double *st_inv;    // 6 per cell: I00 I01 I02 I11 I12 I22 of the symmetric inverse
+    const double *st_wd;     // w * d (3 per c2f entry); null with faces_per_cell (t_wd)
+    const double *st_inv;    // 6 per cell: I00 I01 I02 I11 I12 I22 of the symmetric inverse; null with faces_per_cell (t_inv)
     const int8_t *st_valid;  // per cell
     // optional (the mesh descriptor's edge_nodes): start and end node per edge, and per node its fluid
     // cells in ascending order (mercury::AmbipolarEMF's node lists); null without edge_nodes
     const int32_t *e_nodes;
     const int32_t *n2c_ptr, *n2c_cell;
 };
+
+// The fluid flux through a face (FluxRHS.cpp:41-66): none (Skip kind, or no owned fluid cell), between two cells, or
+// a ghost face whose one fluid cell lies on the L or on the R side of the canonical normal.
+enum FaceFlux { FF_NONE = 0, FF_INTERIOR = 1, FF_INSIDE_L = 2, FF_INSIDE_R = 3 };
 
 constexpr int kMaxValence = 32; // faces per edge handled by the UCT edge kernel (checked at mesh creation)
 
@@ -252,7 +289,8 @@ struct MhdMesh
         cfa_idx;
     mhd::DBuf<int8_t> c2f_sgn, f2e_sgn, e2f_sgn, f2c_sgn, material, face_kind, edge_mode, st_valid, cfa_sgn;
     mhd::DBuf<double> edge_vec, edge_mid, edge_len, face_area, face_center, face_area_mag, cell_center, cell_volume, ec_weight,
-        ef_weight, star1, star2, st_wd, st_inv, st_dx, t_wd, t_dx, t_inv;
+        ef_weight, star1, star2, st_wd, st_inv, st_dx, t_geo, fna, cinv;
+    mhd::DBuf<int4> frec;
     mhd::DBuf<int32_t> t_nb, e_nodes, n2c_ptr, n2c_cell;
     mhd::DBuf<int8_t> t_sg;
     // scratch reused across calls (stream ordered): face fluxes, face EMF candidates, reductions

@@ -103,13 +103,6 @@ __device__ __forceinline__ bool grid_sum32(double v, double *part, unsigned *cou
 // the basis vectors start at i * ldv, which need not be 16-byte aligned.
 constexpr int kGsThreads = 128;
 constexpr int kGsStages = 3; // tiles in flight per block: the one being read and kGsStages - 1 ahead
-__device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
-{
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // Pass 1: h_i = V_i . w (i < NV) into H(i, j), and |w|^2 into red[32], over the owned edges.  red holds 96
 // doubles: [0, 31) the re-orthogonalisation dots, [32] |w|^2 before the update, [64, 96) the last pass's sums.

@@ -6,42 +6,30 @@
 namespace mhd
 {
 // uns::reconstruct_cell_vector (src/uns/geometry/Reconstruct.cpp:8-46): area-weighted least squares
-// b . n_f = flux_f / A_f, the 3x3 normal matrix built and inverted per cell.
+// b . n_f = flux_f / A_f.  The normal matrix depends on the metric alone: its inverse comes from the mesh
+// (MeshView::cinv), and the right-hand side sum (s n)(s flux) is formed as sum n flux (the sign squares away exactly).
 __device__ __forceinline__ V3 cell_vector(const MeshView &m, const double *__restrict__ flux, int32_t c)
 {
-    // the full (not symmetrised) matrix: its two triangles round differently and both enter det
-    double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, r[3] = {0, 0, 0};
-    for (int32_t k = m.c2f_ptr[c]; k < m.c2f_ptr[c + 1]; ++k)
+    double r0 = 0, r1 = 0, r2 = 0;
+    auto add = [&](int32_t f) {
+        const D4 n = ld_d4(m.fna + 4 * (int64_t)f);
+        if (n.w <= 0) return;
+        const double phi = flux[f];
+        r0 += n.x * phi;
+        r1 += n.y * phi;
+        r2 += n.z * phi;
+    };
+    if (m.faces_per_cell == 4)
     {
-        const int32_t f = m.c2f_idx[k];
-        const double A = m.face_area_mag[f];
-        if (A <= 0) continue;
-        const double s = m.c2f_sgn[k];
-        const V3 n = (s / A) * ld3(m.face_area, f);
-        const double nv[3] = {n.x, n.y, n.z};
-        const double phi = s * flux[f];
-        for (int i = 0; i < 3; ++i)
-        {
-            r[i] += nv[i] * phi;
-            for (int j = 0; j < 3; ++j) M[i][j] += A * nv[i] * nv[j];
-        }
+        const int4 f = *reinterpret_cast<const int4 *>(m.c2f_idx + 4 * (int64_t)c);
+        add(f.x); add(f.y); add(f.z); add(f.w);
     }
-    const double det = M[0][0] * (M[1][1] * M[2][2] - M[1][2] * M[2][1]) - M[0][1] * (M[1][0] * M[2][2] - M[1][2] * M[2][0]) +
-                       M[0][2] * (M[1][0] * M[2][1] - M[1][1] * M[2][0]);
-    const double sc = dmax(dmax(dmax(M[0][0], M[1][1]), M[2][2]), 1e-300);
-    if (fabs(det) < 1e-12 * sc * sc * sc) return mk(0, 0, 0);
-    double I[3][3];
-    I[0][0] = (M[1][1] * M[2][2] - M[1][2] * M[2][1]) / det;
-    I[0][1] = (M[0][2] * M[2][1] - M[0][1] * M[2][2]) / det;
-    I[0][2] = (M[0][1] * M[1][2] - M[0][2] * M[1][1]) / det;
-    I[1][0] = (M[1][2] * M[2][0] - M[1][0] * M[2][2]) / det;
-    I[1][1] = (M[0][0] * M[2][2] - M[0][2] * M[2][0]) / det;
-    I[1][2] = (M[0][2] * M[1][0] - M[0][0] * M[1][2]) / det;
-    I[2][0] = (M[1][0] * M[2][1] - M[1][1] * M[2][0]) / det;
-    I[2][1] = (M[0][1] * M[2][0] - M[0][0] * M[2][1]) / det;
-    I[2][2] = (M[0][0] * M[1][1] - M[0][1] * M[1][0]) / det;
-    return mk(I[0][0] * r[0] + I[0][1] * r[1] + I[0][2] * r[2], I[1][0] * r[0] + I[1][1] * r[1] + I[1][2] * r[2],
-              I[2][0] * r[0] + I[2][1] * r[1] + I[2][2] * r[2]);
+    else
+        for (int32_t k = m.c2f_ptr[c]; k < m.c2f_ptr[c + 1]; ++k) add(m.c2f_idx[k]);
+    const int64_t n = m.nc;
+    const double *I = m.cinv + c;
+    return mk(I[0] * r0 + I[n] * r1 + I[2 * n] * r2, I[3 * n] * r0 + I[4 * n] * r1 + I[5 * n] * r2,
+              I[6 * n] * r0 + I[7 * n] * r1 + I[8 * n] * r2);
 }
 
 // (d1^T star2 phi)_e: the resistive current flux of ImplicitInduction::apply_F (ImplicitInduction.cpp:133-137)

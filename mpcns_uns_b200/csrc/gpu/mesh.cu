@@ -85,15 +85,15 @@ __global__ void k_slot_dx(MeshView m, double *dx)
     for (int32_t k = m.c2f_ptr[c]; k < m.c2f_ptr[c + 1]; ++k) st3(dx, k, ld3(m.face_center, m.c2f_idx[k]) - xc);
 }
 
-// structure-of-arrays copy of the stencil of a tetrahedral mesh (4 slots per cell)
-__global__ void k_tet_tables(MeshView m, int32_t *nb, int8_t *sg, double *wd, double *dx, double *inv)
+// structure-of-arrays copy of the stencil of a mesh of nfc-faced cells (4: tetrahedra, 6: hexahedra)
+__global__ void k_slot_tables(MeshView m, int nfc, int32_t *nb, int8_t *sg, double *wd, double *dx, double *inv)
 {
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int64_t n = m.nc;
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < nfc; ++j)
     {
-        const int64_t k = 4 * (int64_t)c + j;
+        const int64_t k = nfc * (int64_t)c + j;
         nb[j * n + c] = c < m.no_cells ? m.st_nb[k] : INT32_MIN;
         sg[j * n + c] = m.c2f_sgn[k];
         for (int a = 0; a < 3; ++a)
@@ -103,6 +103,83 @@ __global__ void k_tet_tables(MeshView m, int32_t *nb, int8_t *sg, double *wd, do
         }
     }
     for (int q = 0; q < 6; ++q) inv[q * n + c] = m.st_inv[6 * (int64_t)c + q];
+}
+
+// the faces' records (MeshView::fna, frec)
+__global__ void k_face_records(MeshView m, double *fna, int4 *frec)
+{
+    const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= m.nf) return;
+    const double A = m.face_area_mag[f];
+    const V3 n = (1.0 / A) * ld3(m.face_area, f);
+    double *o = fna + 4 * (int64_t)f;
+    o[0] = n.x; o[1] = n.y; o[2] = n.z; o[3] = A;
+    auto entry = [&](int32_t c) {
+        if (c < 0) return -1;
+        int32_t k = m.c2f_ptr[c];
+        while (k + 1 < m.c2f_ptr[c + 1] && m.c2f_idx[k] != f) ++k;
+        return k;
+    };
+    const int kind = m.face_kind[f];
+    const int32_t p0 = m.f2c_ptr[f], cnt = m.f2c_ptr[f + 1] - p0;
+    bool any = false;
+    for (int32_t k = p0; k < p0 + cnt; ++k) any |= m.f2c_idx[k] < m.no_cells && m.material[m.f2c_idx[k]] == 0;
+    int4 r = make_int4(0, 0, kind << 4, 0);
+    if (kind != 4 && any)
+    {
+        if (cnt == 2 && kind == 0)
+        {
+            r.x = entry(m.face_L[f]);
+            r.y = entry(m.face_R[f]);
+            r.z |= FF_INTERIOR;
+        }
+        else
+        {
+            // the one fluid cell of a boundary / interface face (FluxRHS.cpp:58-66)
+            int32_t q = p0;
+            if (cnt == 2 && m.material[m.f2c_idx[q]] != 0) ++q;
+            r.x = r.y = entry(m.f2c_idx[q]);
+            r.z |= m.f2c_sgn[q] > 0 ? FF_INSIDE_L : FF_INSIDE_R;
+        }
+    }
+    frec[f] = r;
+}
+
+// the inverse of the cell-field fit's normal matrix (MeshView::cinv): the operations of
+// uns::reconstruct_cell_vector (src/uns/geometry/Reconstruct.cpp:8-46) that depend on the metric alone, in its order
+__global__ void k_cell_inverse(MeshView m, double *cinv)
+{
+    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= m.nc) return;
+    // the full (not symmetrised) matrix: its two triangles round differently and both enter det
+    double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    for (int32_t k = m.c2f_ptr[c]; k < m.c2f_ptr[c + 1]; ++k)
+    {
+        const int32_t f = m.c2f_idx[k];
+        const double A = m.face_area_mag[f];
+        if (A <= 0) continue;
+        const V3 n = (static_cast<double>(m.c2f_sgn[k]) / A) * ld3(m.face_area, f);
+        const double nv[3] = {n.x, n.y, n.z};
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) M[i][j] += A * nv[i] * nv[j];
+    }
+    const double det = M[0][0] * (M[1][1] * M[2][2] - M[1][2] * M[2][1]) - M[0][1] * (M[1][0] * M[2][2] - M[1][2] * M[2][0]) +
+                       M[0][2] * (M[1][0] * M[2][1] - M[1][1] * M[2][0]);
+    const double sc = dmax(dmax(dmax(M[0][0], M[1][1]), M[2][2]), 1e-300);
+    double I[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (!(fabs(det) < 1e-12 * sc * sc * sc))
+    {
+        I[0] = (M[1][1] * M[2][2] - M[1][2] * M[2][1]) / det;
+        I[1] = (M[0][2] * M[2][1] - M[0][1] * M[2][2]) / det;
+        I[2] = (M[0][1] * M[1][2] - M[0][2] * M[1][1]) / det;
+        I[3] = (M[1][2] * M[2][0] - M[1][0] * M[2][2]) / det;
+        I[4] = (M[0][0] * M[2][2] - M[0][2] * M[2][0]) / det;
+        I[5] = (M[0][2] * M[1][0] - M[0][0] * M[1][2]) / det;
+        I[6] = (M[1][0] * M[2][1] - M[1][1] * M[2][0]) / det;
+        I[7] = (M[0][1] * M[2][0] - M[0][0] * M[2][1]) / det;
+        I[8] = (M[0][0] * M[1][1] - M[0][1] * M[1][0]) / det;
+    }
+    for (int q = 0; q < 9; ++q) cinv[q * (int64_t)m.nc + c] = I[q];
 }
 
 std::vector<int32_t> ptr32(const int64_t *p, int64_t rows, const char *what)
@@ -308,9 +385,12 @@ int mhd_gpu_mesh_create(const MhdMeshDesc *d, MhdMesh **out)
             MHD_LAUNCH_CHECK();
         }
         v.st_nb = m->st_nb.p; v.st_wd = m->st_wd.p; v.st_inv = m->st_inv.p; v.st_valid = m->st_valid.p;
-        bool tets = nc > 0;
-        for (int64_t c = 0; c < nc && tets; ++c) tets = c2fp[c + 1] - c2fp[c] == 4;
-        v.faces_per_cell = tets ? 4 : 0;
+        // cells of one kind: 4 (tetrahedra) or 6 faces each
+        int32_t nfc = nc > 0 ? c2fp[1] - c2fp[0] : 0;
+        if (nfc != 4 && nfc != 6) nfc = 0;
+        for (int64_t c = 0; c < nc && nfc; ++c)
+            if (c2fp[c + 1] - c2fp[c] != nfc) nfc = 0;
+        v.faces_per_cell = nfc;
         m->st_dx.alloc(3 * static_cast<size_t>(c2fp[nc]));
         if (nc)
         {
@@ -318,18 +398,30 @@ int mhd_gpu_mesh_create(const MhdMeshDesc *d, MhdMesh **out)
             MHD_LAUNCH_CHECK();
         }
         v.st_dx = m->st_dx.p;
-        if (tets)
+        if (nfc)
         {
-            m->t_nb.alloc(4 * static_cast<size_t>(nc));
-            m->t_sg.alloc(4 * static_cast<size_t>(nc));
-            m->t_wd.alloc(12 * static_cast<size_t>(nc));
-            m->t_dx.alloc(12 * static_cast<size_t>(nc));
-            m->t_inv.alloc(6 * static_cast<size_t>(nc));
-            k_tet_tables<<<grid_for(nc, 256), 256, 0, m->stream>>>(v, m->t_nb.p, m->t_sg.p, m->t_wd.p, m->t_dx.p, m->t_inv.p);
+            m->t_nb.alloc(nfc * static_cast<size_t>(nc));
+            m->t_sg.alloc(nfc * static_cast<size_t>(nc));
+            const size_t rows = 3 * nfc * static_cast<size_t>(nc);
+            m->t_geo.alloc(2 * rows + 6 * static_cast<size_t>(nc));
+            double *wd = m->t_geo.p, *dx = wd + rows, *inv = dx + rows;
+            k_slot_tables<<<grid_for(nc, 256), 256, 0, m->stream>>>(v, nfc, m->t_nb.p, m->t_sg.p, wd, dx, inv);
             MHD_LAUNCH_CHECK();
-            v.t_nb = m->t_nb.p; v.t_sg = m->t_sg.p; v.t_wd = m->t_wd.p; v.t_dx = m->t_dx.p; v.t_inv = m->t_inv.p;
+            v.t_nb = m->t_nb.p; v.t_sg = m->t_sg.p; v.t_wd = wd; v.t_dx = dx; v.t_inv = inv;
         }
+        m->fna.alloc(4 * static_cast<size_t>(nf));
+        m->frec.alloc(static_cast<size_t>(nf));
+        m->cinv.alloc(9 * static_cast<size_t>(nc));
+        if (nf) k_face_records<<<grid_for(nf, 256), 256, 0, m->stream>>>(v, m->fna.p, m->frec.p);
+        if (nc) k_cell_inverse<<<grid_for(nc, 128), 128, 0, m->stream>>>(v, m->cinv.p);
+        MHD_LAUNCH_CHECK();
+        v.fna = m->fna.p; v.frec = m->frec.p; v.cinv = m->cinv.p;
         MHD_CUDA(cudaStreamSynchronize(m->stream));
+        if (nfc) // the slot tables hold the same values
+        {
+            m->st_wd.release(); m->st_inv.release(); m->st_dx.release();
+            v.st_wd = v.st_inv = v.st_dx = nullptr;
+        }
         *out = m;
     });
     if (rc != MHD_OK) delete m;

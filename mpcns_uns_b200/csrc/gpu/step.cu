@@ -368,12 +368,17 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
         if (gp.sw_flux) gp.sw_flux += (int64_t)s0 * m.nf;
         const SField<const double> Wg{st->W.p + (int64_t)s0 * 5 * nc, 5 * nc, 1, nc};
         const SField<double> Gg{st->grad.p, 15 * nc, 1, nc};
+        // face values where the state holds them, with the gradients too while a differentiated run records its
+        // stages (floor_flags); the gradients alone for the first-order scheme, mixed polyhedra and the switch log
+        const bool faces = st->fv.n && !gp.sw_lim && !gp.sw_flux;
         P.begin(KP_GRAD, s);
-        if (st->prm.second_order) launch_limited_gradients(m, gp, Wg, Gg, s);
+        if (faces) launch_face_values(m, gp, Wg, st->floor_flags ? &Gg : nullptr, st->fv.p, s);
+        else if (st->prm.second_order) launch_limited_gradients(m, gp, Wg, Gg, s);
         else MHD_CUDA(cudaMemsetAsync(st->grad.p, 0, (size_t)15 * ng * nc * sizeof(double), s));
         P.end(KP_GRAD, s);
         P.begin(KP_FLUX, s);
-        launch_face_flux(m, gp, Wg, SField<const double>{st->grad.p, 15 * nc, 1, nc}, st->F.p, s);
+        if (faces) launch_face_flux_fv(m, gp, st->fv.p, st->F.p, s);
+        else launch_face_flux(m, gp, Wg, SField<const double>{st->grad.p, 15 * nc, 1, nc}, st->F.p, s);
         P.end(KP_FLUX, s);
         if (m.nc)
         {
@@ -526,8 +531,12 @@ int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *p, MhdState **out)
         st->U0.alloc(5 * nc * st->nsp);
         st->U1.alloc(5 * nc * st->nsp);
         st->W.alloc(5 * nc * st->nsp);
-        st->grad.alloc(15 * nc * st->group);
-        st->F.alloc(5 * nf * st->group);
+        if (p->precision != MHD_PREC_MIXED)
+        {
+            if (p->second_order && m.faces_per_cell) st->fv.alloc(5 * (size_t)m.faces_per_cell * nc * st->group);
+            else st->grad.alloc(15 * nc * st->group);
+            st->F.alloc(5 * nf * st->group);
+        }
         st->phi0.alloc(nf);
         st->phi1.alloc(nf);
         st->phi_add.alloc(nf);
