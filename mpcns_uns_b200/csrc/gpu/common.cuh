@@ -205,6 +205,7 @@ struct MeshView
     const int32_t *cfa_idx;         // c2f rows re-ordered by ascending face id (the reference's scatter order)
     const int8_t *cfa_sgn;
     const int8_t *material, *face_kind, *edge_mode;
+    const int8_t *edge_uct; // edge_mode, with 3 for free edges without a UCT value (no face, no length or no fluid cell)
     const double *edge_vec, *edge_mid, *edge_len;
     const double *face_area, *face_center, *face_area_mag;
     const double *cell_center, *cell_volume;
@@ -287,7 +288,7 @@ struct MhdMesh
     bool own_stream = false;
     mhd::DBuf<int32_t> c2f_ptr, c2f_idx, f2e_ptr, f2e_idx, e2f_ptr, e2f_idx, f2c_ptr, f2c_idx, face_L, face_R, ec_ptr, ec_cell, st_nb,
         cfa_idx;
-    mhd::DBuf<int8_t> c2f_sgn, f2e_sgn, e2f_sgn, f2c_sgn, material, face_kind, edge_mode, st_valid, cfa_sgn;
+    mhd::DBuf<int8_t> c2f_sgn, f2e_sgn, e2f_sgn, f2c_sgn, material, face_kind, edge_mode, edge_uct, st_valid, cfa_sgn;
     mhd::DBuf<double> edge_vec, edge_mid, edge_len, face_area, face_center, face_area_mag, cell_center, cell_volume, ec_weight,
         ef_weight, star1, star2, st_wd, st_inv, st_dx, t_geo, fna, cinv;
     mhd::DBuf<int4> frec;

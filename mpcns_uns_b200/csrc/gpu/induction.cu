@@ -190,26 +190,29 @@ void build_edge_face_geo(const MeshView &m, double *geo, cudaStream_t s)
     MHD_LAUNCH_CHECK();
 }
 
-// edge_uct from the per-slot geometry table, for edges of at most kGeoCells cells and kGeoSlots faces: the
-// cells' velocities are staged once in this thread's column of shared memory (su[(3 * k + a) * 128 + lane]),
-// and the face loop runs twice, the second pass forming each face's upwind terms again from the table instead of
-// holding them, so that no per-face array lives in registers.  Every value and every sum is formed by
-// the operations of edge_uct in its order: the results are the same bits.
+// edge_uct from the per-slot geometry table, for edges of at most kGeoCells cells and kGeoSlots faces (and whose
+// MeshView::edge_uct says that the UCT applies), in three loops over the faces:
+//   A  a_ef = max |u . m| over the edge's cells, whose velocities are staged once in this thread's column of shared
+//      memory (su[(3 * k + a) * 128]); the a_ef stay in registers;
+//   B  the central part and the sums of the 2x2 solve; (q.e1, q.e2, sigma) of each face replace the velocities in the
+//      column;
+//   C  the upwind part from them.
+// So a face's geometry is read once and nothing is formed twice.  Every value and every sum is formed by the operations
+// of edge_uct in its order: the results are the same bits.  Latency bound (35% of the warp slots, 46% of the DRAM peak):
+// 2.08M tetrahedral edges 318 us a launch against 420 with the a_ef and q formed again in a second loop over the table;
+// 4 or 5 blocks per SM, which need no spills, 383 and 325.
 constexpr int kGeoCells = 8;
 // pa: phi_ind / |A| per face (k_face_candidate's pa)
 template <bool LOG>
-__device__ __forceinline__ bool edge_uct_geo(const MeshView &m, int32_t e, const double *__restrict__ Ef, const double *__restrict__ u,
-                                             const double *__restrict__ pa, double cuct, const double *__restrict__ geo,
-                                             double *__restrict__ su, double &out, uint32_t *code)
+__device__ __forceinline__ double edge_uct_geo(const MeshView &m, int32_t e, const double *__restrict__ Ef, const double *__restrict__ u,
+                                               const double *__restrict__ pa, double cuct, const double *__restrict__ geo,
+                                               double *__restrict__ su, uint32_t *code)
 {
+    static_assert(kGeoSlots <= kGeoCells, "a face's three values share the columns of the cells");
     const int32_t f0 = m.e2f_ptr[e], nf = m.e2f_ptr[e + 1] - f0;
+    const int32_t q0 = m.ec_ptr[e], nce = m.ec_ptr[e + 1] - q0;
     const double L = m.edge_len[e];
-    if (nf == 0 || L <= 0) return false;
-    const int32_t q0 = m.ec_ptr[e], q1 = m.ec_ptr[e + 1];
-    bool any_fluid = false;
-    for (int32_t k = q0; k < q1 && !any_fluid; ++k) any_fluid = m.material[m.ec_cell[k]] == 0;
-    if (!any_fluid) return false;
-    const int nce = q1 - q0;
+    const V3 t = ld3(m.edge_vec, e);
     // unrolled over the bound so that every cell's id and velocity loads are in flight together
 #pragma unroll
     for (int k = 0; k < kGeoCells; ++k)
@@ -220,16 +223,22 @@ __device__ __forceinline__ bool edge_uct_geo(const MeshView &m, int32_t e, const
             su[(3 * k + 1) * 128] = uk.y;
             su[(3 * k + 2) * 128] = uk.z;
         }
-    const V3 t = ld3(m.edge_vec, e);
-    const V3 th = (1.0 / L) * t;
-    // plane basis (IdealEMF.cpp:14-20)
-    const V3 ax = fabs(th.x) < 0.9 ? mk(1, 0, 0) : mk(0, 1, 0);
-    V3 e1 = cross(th, ax);
-    e1 = (1.0 / sqrt(dot(e1, e1))) * e1;
-    const V3 e2 = cross(th, e1);
-    // the face's largest |u . m| over the edge's cells (and, logged, which cell and its sign)
-    auto a_ef = [&](V3 mi) {
-        double a = 0;
+    const int64_t ne = m.ne;
+    const double *g = geo + e; // component c of slot i at g[(8 * c + i) * ne]
+    // the face ids of the row, loaded together
+    int32_t fid[kGeoSlots];
+#pragma unroll
+    for (int i = 0; i < kGeoSlots; ++i) fid[i] = i < nf ? m.e2f_idx[f0 + i] : 0;
+    double a[kGeoSlots];
+    auto dir = [&](int i) { return mk(g[i * ne], g[(8 + i) * ne], g[(16 + i) * ne]); };
+    V3 m_next = dir(0); // each loop loads the next face's values before it works on the current ones
+#pragma unroll
+    for (int i = 0; i < kGeoSlots; ++i)
+    {
+        if (i >= nf) break;
+        const V3 mi = m_next;
+        if (i + 1 < kGeoSlots && i + 1 < nf) m_next = dir(i + 1);
+        double am = 0;
         int ka = 31;
         bool neg = false;
 #pragma unroll
@@ -237,46 +246,51 @@ __device__ __forceinline__ bool edge_uct_geo(const MeshView &m, int32_t e, const
         {
             if (k >= nce) break;
             const double d = dot(mk(su[(3 * k) * 128], su[(3 * k + 1) * 128], su[(3 * k + 2) * 128]), mi);
-            if (LOG && a < fabs(d))
+            if (LOG && am < fabs(d))
             {
                 ka = k;
                 neg = d < 0;
             }
-            a = dmax(a, fabs(d));
+            am = dmax(am, fabs(d));
         }
+        a[i] = am;
         if (LOG) *code = sw_step(*code, uint32_t(ka & 31) | (neg ? 32u : 0u));
-        return a;
-    };
+    }
     struct Face
     {
-        V3 mi, nrm;
+        V3 nrm, E;
         double sg, w;
     };
-    const int64_t ne = m.ne;
-    auto face = [&](int32_t i) {
-        const double *g = geo + i * ne + e;
-        return Face{mk(g[0], g[8 * ne], g[16 * ne]), mk(g[24 * ne], g[32 * ne], g[40 * ne]), g[48 * ne], g[56 * ne]};
+    auto face = [&](int i) {
+        return Face{mk(g[(24 + i) * ne], g[(32 + i) * ne], g[(40 + i) * ne]), ld3(Ef, fid[i]), g[(48 + i) * ne], g[(56 + i) * ne]};
     };
+    Face f_next = face(0);
+    const V3 th = (1.0 / L) * t;
+    // plane basis (IdealEMF.cpp:14-20)
+    const V3 ax = fabs(th.x) < 0.9 ? mk(1, 0, 0) : mk(0, 1, 0);
+    V3 e1 = cross(th, ax);
+    e1 = (1.0 / sqrt(dot(e1, e1))) * e1;
+    const V3 e2 = cross(th, e1);
     double Ec = 0, M11 = 0, M12 = 0, M22 = 0, g1 = 0, g2 = 0;
-    // the face ids of the row, loaded together
-    int32_t fid[kGeoSlots];
 #pragma unroll
-    for (int i = 0; i < kGeoSlots; ++i) fid[i] = i < nf ? m.e2f_idx[f0 + i] : 0;
-#pragma unroll
-    for (int32_t i = 0; i < kGeoSlots; ++i)
+    for (int i = 0; i < kGeoSlots; ++i)
     {
         if (i >= nf) break;
-        const int32_t f = fid[i];
-        const Face F = face(i);
-        Ec += F.w * dot(ld3(Ef, f), t);
-        const double a = a_ef(F.mi);
-        const V3 qv = (a * F.sg) * F.nrm;
+        const Face F = f_next;
+        if (i + 1 < kGeoSlots && i + 1 < nf) f_next = face(i + 1);
+        const V3 nrm = F.nrm;
+        const double sg = F.sg, w = F.w;
+        Ec += w * dot(F.E, t);
+        const V3 qv = (a[i] * sg) * nrm;
         const double qa = dot(qv, e1), qb = dot(qv, e2);
-        M11 += F.w * qa * qa;
-        M12 += F.w * qa * qb;
-        M22 += F.w * qb * qb;
-        g1 += F.w * qa;
-        g2 += F.w * qb;
+        su[(3 * i) * 128] = qa;
+        su[(3 * i + 1) * 128] = qb;
+        su[(3 * i + 2) * 128] = sg;
+        M11 += w * qa * qa;
+        M12 += w * qa * qb;
+        M22 += w * qb * qb;
+        g1 += w * qa;
+        g2 += w * qb;
     }
     const double tr = M11 + M22;
     const double eps = 1e-14 * tr;
@@ -288,27 +302,22 @@ __device__ __forceinline__ bool edge_uct_geo(const MeshView &m, int32_t e, const
         l1 = ((M22 + eps) * g1 - M12 * g2) / det;
         l2 = ((M11 + eps) * g2 - M12 * g1) / det;
     }
-    double Eu = 0;
+    double Eu = 0, w_next = g[56 * ne], p_next = pa[fid[0]];
 #pragma unroll
-    for (int32_t i = 0; i < kGeoSlots; ++i)
+    for (int i = 0; i < kGeoSlots; ++i)
     {
         if (i >= nf) break;
-        const int32_t f = fid[i];
-        const Face F = face(i);
-        double a = 0;
-#pragma unroll
-        for (int k = 0; k < kGeoCells; ++k)
+        const double w = w_next, ph = p_next;
+        if (i + 1 < kGeoSlots && i + 1 < nf)
         {
-            if (k >= nce) break;
-            a = dmax(a, fabs(dot(mk(su[(3 * k) * 128], su[(3 * k + 1) * 128], su[(3 * k + 2) * 128]), F.mi)));
+            w_next = g[(57 + i) * ne];
+            p_next = pa[fid[i + 1]];
         }
-        const V3 qv = (a * F.sg) * F.nrm;
-        const double qa = dot(qv, e1), qb = dot(qv, e2);
-        const double omega = F.w * (1.0 - (qa * l1 + qb * l2));
-        Eu += omega * a * F.sg * pa[f];
+        const double qa = su[(3 * i) * 128], qb = su[(3 * i + 1) * 128], sg = su[(3 * i + 2) * 128];
+        const double omega = w * (1.0 - (qa * l1 + qb * l2));
+        Eu += omega * a[i] * sg * ph;
     }
-    out = Ec + 2.0 * cuct * L * Eu;
-    return true;
+    return Ec + 2.0 * cuct * L * Eu;
 }
 
 template <int MAXV>
@@ -340,17 +349,18 @@ __global__ void __launch_bounds__(128, GEO ? 6 : 4) k_edge_emf_assign(MeshView m
     double val = 0.0;
     if (e < m.no_edges)
     {
-        const int mode = m.edge_mode[e];
+        const int mode = GEO ? m.edge_uct[e] : m.edge_mode[e];
         if (mode == 1) val = 0.0;
         else if (mode == 2) val = dot(E_inf, ld3(m.edge_vec, e));
         else
         {
             double v;
             uint32_t code = 0;
-            bool ok;
-            if constexpr (GEO) ok = edge_uct_geo<LOG>(m, e, Ef, u, pa, cuct, geo, su + threadIdx.x, v, &code);
-            else ok = edge_uct<MAXV, LOG>(m, e, Ef, u, phi_ind, cuct, v, &code);
-            if (ok) val += v;
+            if constexpr (GEO)
+            {
+                if (mode == 0) val += edge_uct_geo<LOG>(m, e, Ef, u, pa, cuct, geo, su + threadIdx.x, &code);
+            }
+            else if (edge_uct<MAXV, LOG>(m, e, Ef, u, phi_ind, cuct, v, &code)) val += v;
             if (LOG) sw_log(sw, e, code);
             // AmbipolarEMF::add (Ambipolar.cpp:69-87) after the ideal EMF; on wall and inflow edges the
             // reference overwrites it with the boundary value

@@ -145,6 +145,21 @@ __global__ void k_face_records(MeshView m, double *fna, int4 *frec)
     frec[f] = r;
 }
 
+// MeshView::edge_uct: IdealEMF.cpp:59-70 skips edges without faces, length or a fluid cell
+__global__ void k_edge_uct_kind(MeshView m, int8_t *kind)
+{
+    const int32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m.ne) return;
+    int k = m.edge_mode[e];
+    if (k != 1 && k != 2)
+    {
+        bool fluid = false;
+        for (int32_t q = m.ec_ptr[e]; q < m.ec_ptr[e + 1]; ++q) fluid |= m.material[m.ec_cell[q]] == 0;
+        k = fluid && m.edge_len[e] > 0 && m.e2f_ptr[e + 1] > m.e2f_ptr[e] ? 0 : 3;
+    }
+    kind[e] = static_cast<int8_t>(k);
+}
+
 // the inverse of the cell-field fit's normal matrix (MeshView::cinv): the operations of
 // uns::reconstruct_cell_vector (src/uns/geometry/Reconstruct.cpp:8-46) that depend on the metric alone, in its order
 __global__ void k_cell_inverse(MeshView m, double *cinv)
@@ -412,6 +427,9 @@ int mhd_gpu_mesh_create(const MhdMeshDesc *d, MhdMesh **out)
         m->fna.alloc(4 * static_cast<size_t>(nf));
         m->frec.alloc(static_cast<size_t>(nf));
         m->cinv.alloc(9 * static_cast<size_t>(nc));
+        m->edge_uct.alloc(static_cast<size_t>(ne));
+        v.edge_uct = m->edge_uct.p;
+        if (ne) k_edge_uct_kind<<<grid_for(ne, 256), 256, 0, m->stream>>>(v, m->edge_uct.p);
         if (nf) k_face_records<<<grid_for(nf, 256), 256, 0, m->stream>>>(v, m->fna.p, m->frec.p);
         if (nc) k_cell_inverse<<<grid_for(nc, 128), 128, 0, m->stream>>>(v, m->cinv.p);
         MHD_LAUNCH_CHECK();
