@@ -21,7 +21,8 @@
 //     restarts up to 31; beyond, each modified Gram-Schmidt subtraction w -= H(i-1, j) V_{i-1} is fused
 //     with the next dot w . V_i, consecutive passes sweeping the edges in opposite directions so that the
 //     tail of w and V_{i-1} left in L2 is reused first;
-//   * every dot finishes in the kernel that produces it (the last block adds the block partials), and
+//   * every dot of the operator finishes in the kernel that produces it (the last block adds the block partials), those
+//     of Gram-Schmidt in k_cgs_tail, which also rotates the column, and
 //     a restart cycle runs as one CUDA graph whose steps test a device-side flag, so the host waits
 //     once per restart instead of once per Arnoldi step.
 #include <array>
@@ -132,6 +133,7 @@ __global__ void k_to_float(const double *a, float *b, int64_t n)
 
 __global__ void k_ind_s2phi(MeshView m, const double *__restrict__ phi, double *__restrict__ s2phi)
 {
+    pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f < m.nf) s2phi[f] = m.star2[f] * phi[f];
 }
@@ -144,6 +146,7 @@ __global__ void k_ind_hall(MeshView m, Gate gt, const int32_t *__restrict__ slot
                            const double *__restrict__ b, const double *__restrict__ alpha, const double *__restrict__ B0,
                            double *__restrict__ g)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.no_cells || gt.off()) return;
     if (alpha[c] == 0.0 || m.material[c] != 0)
@@ -171,6 +174,7 @@ __global__ void k_ind_hall(MeshView m, Gate gt, const int32_t *__restrict__ slot
 __global__ void __launch_bounds__(256) k_dot(const double *__restrict__ a, const double *__restrict__ b, int32_t n, double *part,
                                              unsigned *counter, int op, double *out)
 {
+    pdl_begin();
     double s = 0.0;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += a[i] * b[i];
     grid_sum_tail(s, part, counter, op, out);
@@ -222,6 +226,7 @@ __global__ void __launch_bounds__(256) k_mgs(Gate gt, double *__restrict__ w, co
 
 __global__ void k_vec_x0(int32_t n, const double *Ee, const double *corr, const int8_t *dir, double *x0, double *delta)
 {
+    pdl_begin();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     x0[i] = (corr && !dir[i]) ? Ee[i] + corr[i] : Ee[i];
@@ -229,12 +234,14 @@ __global__ void k_vec_x0(int32_t n, const double *Ee, const double *corr, const 
 }
 __global__ void k_vec_add(int32_t n, const double *a, const double *b, double *c)
 {
+    pdl_begin();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) c[i] = a[i] + b[i];
 }
 // r = dir ? 0 : b - Ax
 __global__ void k_vec_resid(int32_t n, const double *b, const double *Ax, const int8_t *dir, double *r)
 {
+    pdl_begin();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) r[i] = dir[i] ? 0.0 : b[i] - Ax[i];
 }
@@ -243,6 +250,7 @@ __global__ void k_vec_resid(int32_t n, const double *b, const double *Ax, const 
 __global__ void k_vec_pd(int32_t n, double dt, const double *dte, const double *mc, const double *d2, const int8_t *dir, double *pd,
                          int8_t *dirc)
 {
+    pdl_begin();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     pd[i] = dir[i] ? 0.0 : 1.0 / (1.0 + (dte ? dte[i] : dt) * mc[i] * d2[i]);
@@ -251,6 +259,7 @@ __global__ void k_vec_pd(int32_t n, double dt, const double *dte, const double *
 // V0 = r / beta, and the face pass's input V0 * pd
 __global__ void k_vec_v0(int32_t n, const double *r, const double *beta, double *V0, const double *pd, double *zs, float *zs32)
 {
+    pdl_begin();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double v = r[i] / *beta;
@@ -262,6 +271,7 @@ __global__ void k_vec_v0(int32_t n, const double *r, const double *beta, double 
 // start of a restart cycle: g = (beta, 0, ...), at most `limit` Arnoldi steps, early exit at |g_{j+1}| <= tol
 __global__ void k_cycle_init(Ctl *ctl, int limit, double tol, double dt, double *g, int n, const double *beta)
 {
+    pdl_begin();
     ctl->done = 0;
     ctl->jend = 0;
     ctl->limit = limit;
@@ -297,6 +307,126 @@ __global__ void k_givens(Ctl *ctl, double *H, int mcols, int j, double *cs, doub
     if (fabs(g[j + 1]) <= ctl->tol) ctl->done = 1;
 }
 
+// The sums of a Gram-Schmidt pass from its blocks' rows of partial sums, and what they decide.
+//   pass 0: the dots H(0..j, j) and |w|^2 (red[32]);
+//   pass 1: if the subtraction cancelled (|w|^2 < |w_before|^2 / 2) and the remaining components s along the basis are
+//           above round-off (|s| > 1e-12 |w|), s goes to red[0..j] and ctl->reorth asks for pass 2; else the column is
+//           complete with H(j+1, j) = |w|;
+//   pass 2: adds red[0..j] to H(:, j) and completes the column.
+// A complete column gets its Givens rotations and the early-exit test (:337-347) from the warp that has it.
+// One block: the rows are added along 16 chains per value, warp (k, u) the rows k + 4u + 16i in order, so the order of
+// the sums is fixed, and a chain's loads are issued 16 at a time.  Separate from the pass: there its last block added
+// the rows with four warps and four loads in flight, 18-20 us of a 25 us pass over 263k edges; here 3.7 us.
+__global__ void __launch_bounds__(512) k_cgs_tail(Gate gt, Ctl *ctl, int pass, int j, int grid, int rows, const double *__restrict__ part,
+                                                  double *red, double *H, int mcols, double *gcs, double *gsn, double *g, double *nrm)
+{
+    pdl_begin();
+    if (gt.off() || (pass == 2 && !ctl->reorth)) return;
+    __shared__ double sh[16][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = w & 3, u = w >> 2;
+    const int groups = grid - 12 > k ? (grid - 13 - k) / 16 + 1 : 0; // whole groups of 16 rows that hold row k + 12
+    double a = 0.0;
+    constexpr int U = 16;
+    for (int i0 = 0; i0 < groups && k + 4 * u + 16 * i0 < rows; i0 += U)
+    {
+        double v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+        {
+            const int b = k + 4 * u + 16 * (i0 + q);
+            v[q] = i0 + q < groups && b < rows ? __ldcg(part + (int64_t)b * 32 + lane) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) a += v[q];
+    }
+    if (u == 0)
+        for (int b = k + 16 * groups; b < grid && b < rows; b += 4) a += __ldcg(part + (int64_t)b * 32 + lane);
+    sh[w][lane] = a;
+    __syncthreads();
+    if (w) return;
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s += (sh[q][lane] + sh[q + 4][lane]) + (sh[q + 8][lane] + sh[q + 12][lane]);
+    if (pass == 0)
+    {
+        if (lane <= j) H[lane * mcols + j] = s;
+        if (lane == 31) red[32] = s;
+        return;
+    }
+    const double nn = __shfl_sync(0xffffffffu, s, 31), sl = lane <= j ? s : 0.0;
+    double ss = sl * sl;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (pass == 1 && nn < 0.5 * red[32] && ss > 1e-24 * nn)
+    {
+        if (lane <= j) red[lane] = sl;
+        if (lane == 0)
+        {
+            ctl->reorth = 1;
+            ++ctl->n_reorth;
+        }
+        return;
+    }
+    double h = lane <= j ? H[lane * mcols + j] : 0.0;
+    if (pass == 2 && lane <= j) h += red[lane];
+    const double c_l = lane < j ? gcs[lane] : 0.0, s_l = lane < j ? gsn[lane] : 0.0, hn = sqrt(nn);
+    double cur = __shfl_sync(0xffffffffu, h, 0);
+    for (int i = 0; i < j; ++i)
+    {
+        const double c = __shfl_sync(0xffffffffu, c_l, i), sn = __shfl_sync(0xffffffffu, s_l, i), nx = __shfl_sync(0xffffffffu, h, i + 1);
+        const double t = c * cur + sn * nx;
+        cur = -sn * cur + c * nx;
+        if (lane == i) h = t;
+    }
+    if (lane < j) H[lane * mcols + j] = h;
+    if (lane) return;
+    nrm[j + 1] = hn; // H(j+1, j) before the rotation: the divisor of V_{j+1}
+    const double den = hypot(cur, hn), cs = den > 0 ? cur / den : 1.0, sn = den > 0 ? hn / den : 0.0, gj = g[j], gn = -sn * gj;
+    H[j * mcols + j] = den;
+    H[(j + 1) * mcols + j] = 0.0;
+    gcs[j] = cs;
+    gsn[j] = sn;
+    g[j + 1] = gn;
+    g[j] = cs * gj;
+    ctl->jend = j + 1;
+    ctl->reorth = 0;
+    if (fabs(gn) <= ctl->tol) ctl->done = 1;
+}
+
+// The back substitution below for at most 32 steps by one warp: lane i holds row i and forms its product with every y_k as
+// soon as that is known; only the subtractions, in the row's order, are left to the serial chain.  The same operations in
+// the same order (30 steps: 32 us by one thread with the triangle in global memory).
+__global__ void __launch_bounds__(32) k_backsub_warp(const Ctl *ctl, const double *H, int mcols, const double *g, double *y, double *jend_out)
+{
+    pdl_begin();
+    const int j = ctl->jend, l = threadIdx.x;
+    const double gl = l < j ? g[l] : 0.0;
+    double row[32], s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) row[k] = l <= k && k < j ? H[l * mcols + k] : 0.0;
+#pragma unroll
+    for (int i = 31; i >= 0; --i)
+    {
+        if (i >= j) continue;
+        if (l == i)
+        {
+            s = gl;
+#pragma unroll
+            for (int k = i + 1; k < 32; ++k)
+                if (k < j) s -= row[k];
+            s = s / row[i];
+            y[i] = s;
+        }
+        const double yi = __shfl_sync(0xffffffffu, s, i);
+        if (l < i) row[i] = row[i] * yi;
+    }
+    if (l == 0)
+    {
+        jend_out[0] = j;
+        jend_out[1] = ctl->n_reorth;
+    }
+}
+
 // back substitution of the least-squares problem (:349-354) over the jend steps of the cycle; single thread
 __global__ void k_backsub(const Ctl *ctl, const double *H, int mcols, const double *g, double *y, double *jend_out)
 {
@@ -315,6 +445,7 @@ __global__ void k_backsub(const Ctl *ctl, const double *H, int mcols, const doub
 __global__ void k_vec_update(const Ctl *ctl, int32_t n, const double *V, const double *y, const double *pd, const int8_t *dir,
                              const double *x0, double *delta, double *z)
 {
+    pdl_begin();
     const int32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const int j = ctl->jend;
@@ -349,6 +480,7 @@ __global__ void k_vec_addz(int32_t n, const double *pz, const double *x0, double
 // E = x0 + delta, corr = dir ? 0 : E - E_expl (:379-381)
 __global__ void k_vec_final(int32_t n, const double *x0, const double *delta, const double *Ee, const int8_t *dir, double *E, double *corr)
 {
+    pdl_begin();
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double v = x0[i] + delta[i];
@@ -375,16 +507,16 @@ void op64(MhdInduction *I, const MatIn &in, const double *phi_in, double dt, dou
     if (in.x || in.src)
     {
         if (m.nf)
-            IND_LAUNCH(I, KI_FACE, s, (m.tri_faces ? k_ind_face<double, true> : k_ind_face<double, false>)<<<g1(m.nf), 256, 0, s>>>(
-                                          m, fz.gt, in, hall || ideal, resistive, I->phi.p, I->s2phi.p));
+            IND_LAUNCH(I, KI_FACE, s, launch_pdl(m.tri_faces ? k_ind_face<double, true> : k_ind_face<double, false>, g1(m.nf), 256, 0, s, m, fz.gt, in,
+                                              hall || ideal, resistive, I->phi.p, I->s2phi.p));
         phi = I->phi.p;
     }
     else if (resistive && m.nf)
-        IND_LAUNCH(I, KI_FACE, s, k_ind_s2phi<<<g1(m.nf), 256, 0, s>>>(m, phi, I->s2phi.p));
+        IND_LAUNCH(I, KI_FACE, s, launch_pdl(k_ind_s2phi, g1(m.nf), 256, 0, s, m, phi, I->s2phi.p));
     // the cell field from the face fluxes (:138-149), for the Hall and the ideal parts
     if ((hall || ideal) && m.nc)
-        IND_LAUNCH(I, KI_BCELL, s, (m.faces_per_cell == 4 ? k_ind_bcell<double, true> : k_ind_bcell<double, false>)<<<g1(m.nc), 256, 0, s>>>(
-                                       m, fz.gt, I->recon.p, phi, I->bcell.p));
+        IND_LAUNCH(I, KI_BCELL, s, launch_pdl(m.faces_per_cell == 4 ? k_ind_bcell<double, true> : k_ind_bcell<double, false>, g1(m.nc), 256, 0, s, m,
+                                           fz.gt, I->recon.p, phi, I->bcell.p));
     // the ideal EMF of the frozen velocities and the cell field of phi (:150-158); masked in the edge pass
     if (ideal && m.ne)
     {
@@ -395,8 +527,8 @@ void op64(MhdInduction *I, const MatIn &in, const double *phi_in, double dt, dou
     }
     if (hall && m.nc && m.no_cells)
         IND_LAUNCH(I, KI_HALL, s,
-                   (m.faces_per_cell == 4 ? k_ind_hall<true> : k_ind_hall<false>)<<<g1(m.no_cells), 256, 0, s>>>(m, fz.gt, I->slot_nb.p, I->slot_sa.p, I->bcell.p, I->alpha.p, I->B0.p,
-                                                                 I->g.p));
+                   launch_pdl(m.faces_per_cell == 4 ? k_ind_hall<true> : k_ind_hall<false>, g1(m.no_cells), 256, 0, s, m, fz.gt, I->slot_nb.p,
+                              I->slot_sa.p, I->bcell.p, I->alpha.p, I->B0.p, I->g.p));
     EdgeArgs<double> a;
     a.resistive = resistive; a.hall = hall;
     if (ideal)
@@ -407,7 +539,8 @@ void op64(MhdInduction *I, const MatIn &in, const double *phi_in, double dt, dou
     a.s2phi = I->s2phi.p; a.g = I->g.p; a.mcoef = I->mcoef.p; a.ecw = m.ec_weight; a.tvec = m.edge_vec;
     a.in = in; a.dt = dt; a.dtp = fz.dtp; a.vout = fz.vout; a.dir = fz.dir; a.v0 = fz.v0; a.dot = fz.dot; a.gt = fz.gt;
     a.part = I->part.p; a.counter = I->counter.p; a.out = y;
-    if (m.ne) IND_LAUNCH(I, KI_EDGE, s, (m.max_valence <= 8 && m.max_edge_cells <= 8 ? k_ind_edge<double, 8> : k_ind_edge<double, 0>)<<<I->edge_blocks, 256, 0, s>>>(m, a));
+    if (m.ne) IND_LAUNCH(I, KI_EDGE, s, launch_pdl(m.max_valence <= 8 && m.max_edge_cells <= 8 ? k_ind_edge<double, 8> : k_ind_edge<double, 0>,
+                                                 I->edge_blocks, 256, 0, s, m, a));
 }
 
 void apply_plain(MhdInduction *I, const double *x, double dt, double *y, const double *dte = nullptr)
@@ -422,7 +555,7 @@ void apply_plain(MhdInduction *I, const double *x, double dt, double *y, const d
 void dev_dot(MhdInduction *I, const double *a, const double *b, int op, double *out)
 {
     cudaStream_t s = I->mesh->stream;
-    IND_LAUNCH(I, KI_VECTOR, s, k_dot<<<kRedBlocks, 256, 0, s>>>(a, b, I->mesh->v.no_edges, I->part.p, I->counter.p, op, out));
+    IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_dot, kRedBlocks, 256, 0, s, a, b, I->mesh->v.no_edges, I->part.p, I->counter.p, op, out));
 }
 
 // The mr Arnoldi steps of one restart cycle (:333-348), each gated by the cycle control:
@@ -470,10 +603,16 @@ void enqueue_cycle(MhdInduction *I)
         else op64(I, in, nullptr, 0.0, I->w.p, fz);
         if (cgs)
         {
-            CgsArgs ca{gt, I->ctl.p, I->w.p, V, ne, ne, m.no_edges, I->part.p, I->red.p, H, I->counter.p, mr, I->pd.p,
+            CgsArgs ca{gt, I->ctl.p, I->w.p, V, ne, ne, m.no_edges, I->part.p, I->red.p, H, mr, I->pd.p,
                        I->mixed ? nullptr : I->zs.p, I->mixed ? I->zs32.p : nullptr};
-            for (int pass = 0; pass < 3; ++pass) IND_LAUNCH(I, KI_MGS, s, cgs_launch(j, ca, I->cgs_grid + 2 * j, s, pass));
-            IND_LAUNCH(I, KI_SCALAR, s, k_givens<<<1, 1, 0, s>>>(I->ctl.p, H, mr, j, I->cs.p, I->sn.p, I->gv.p, I->nrm.p));
+            for (int pass = 0; pass < 3; ++pass)
+            {
+                const int grid = I->cgs_grid[2 * j + (pass ? 1 : 0)];
+                IND_LAUNCH(I, KI_MGS, s, cgs_launch(j, ca, I->cgs_grid + 2 * j, s, pass));
+                IND_LAUNCH(I, KI_SCALAR, s, launch_pdl(k_cgs_tail, 1, 512, 0, s, gt, I->ctl.p, pass, j, grid,
+                                                       std::min(grid, cgs_tiles(pass ? ne : m.no_edges)), I->part.p, I->red.p, H, mr, I->cs.p,
+                                                       I->sn.p, I->gv.p, I->nrm.p));
+            }
             continue;
         }
         for (int i = 1; i <= j + 1; ++i)
@@ -562,12 +701,12 @@ int solve_impl(MhdInduction *I, const double *Phi, const double *Ee, const int8_
         if (!warm) I->have_corr = false;
         I->last_reorth = 0;
         double *sc = I->scal.p; // [0] |b|  [1] beta  [2] steps of the last cycle
-        IND_LAUNCH(I, KI_VECTOR, s, k_vec_x0<<<ge, 256, 0, s>>>(ne, Ee, I->have_corr ? I->corr.p : nullptr, dir, I->x0.p, I->delta.p));
+        IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_vec_x0, ge, 256, 0, s, ne, Ee, I->have_corr ? I->corr.p : nullptr, dir, I->x0.p, I->delta.p));
         op64(I, MatIn{}, Phi, 0.0, I->Fn.p);                                                      // F(Phi^n)
-        IND_LAUNCH(I, KI_VECTOR, s, k_vec_add<<<ge, 256, 0, s>>>(ne, Ee, I->Fn.p, I->b.p));     // b = E_expl + F(Phi^n)
+        IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_vec_add, ge, 256, 0, s, ne, Ee, I->Fn.p, I->b.p));     // b = E_expl + F(Phi^n)
         apply_plain(I, I->x0.p, dtA, I->Ax.p, dte);                                               // A x0
-        IND_LAUNCH(I, KI_VECTOR, s, k_vec_resid<<<ge, 256, 0, s>>>(ne, I->b.p, I->Ax.p, dir, I->r.p));
-        IND_LAUNCH(I, KI_VECTOR, s, k_vec_pd<<<ge, 256, 0, s>>>(ne, dt, dte, I->mcoef.p, I->d2.p, dir, I->pd.p, I->dirc.p));
+        IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_vec_resid, ge, 256, 0, s, ne, I->b.p, I->Ax.p, dir, I->r.p));
+        IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_vec_pd, ge, 256, 0, s, ne, dt, dte, I->mcoef.p, I->d2.p, dir, I->pd.p, I->dirc.p));
         if (I->mode == 2) ilu_factor(I, dt, dir); // (:317-318)
         dev_dot(I, I->b.p, I->b.p, 2, sc + 0);
         dev_dot(I, I->r.p, I->r.p, 1, sc + 1);
@@ -580,10 +719,10 @@ int solve_impl(MhdInduction *I, const double *Phi, const double *Ee, const int8_
         while (beta > tol && total < I->p.max_it)
         {
             IND_LAUNCH(I, KI_VECTOR, s,
-                       k_vec_v0<<<ge, 256, 0, s>>>(ne, I->r.p, sc + 1, I->V.p, I->pd.p, I->mixed ? nullptr : I->zs.p,
+                       launch_pdl(k_vec_v0, ge, 256, 0, s, ne, I->r.p, sc + 1, I->V.p, I->pd.p, I->mixed ? nullptr : I->zs.p,
                                                    I->mixed ? I->zs32.p : nullptr));
             IND_LAUNCH(I, KI_SCALAR, s,
-                       k_cycle_init<<<1, 1, 0, s>>>(I->ctl.p, std::min(mr, I->p.max_it - total), tol, dtA, I->gv.p, mr + 1, sc + 1));
+                       launch_pdl(k_cycle_init, 1, 1, 0, s, I->ctl.p, std::min(mr, I->p.max_it - total), tol, dtA, I->gv.p, mr + 1, sc + 1));
             if (!I->prof.on && !I->cycle_tried[I->mode]) build_cycle_graph(I);
             if (!I->prof.on && I->cycle[I->mode])
             {
@@ -592,7 +731,8 @@ int solve_impl(MhdInduction *I, const double *Phi, const double *Ee, const int8_
             }
             else
                 enqueue_cycle(I);
-            IND_LAUNCH(I, KI_SCALAR, s, k_backsub<<<1, 1, 0, s>>>(I->ctl.p, I->H.p, mr, I->gv.p, I->yv.p, sc + 2));
+            if (mr <= 32) IND_LAUNCH(I, KI_SCALAR, s, launch_pdl(k_backsub_warp, 1, 32, 0, s, I->ctl.p, I->H.p, mr, I->gv.p, I->yv.p, sc + 2));
+            else IND_LAUNCH(I, KI_SCALAR, s, k_backsub<<<1, 1, 0, s>>>(I->ctl.p, I->H.p, mr, I->gv.p, I->yv.p, sc + 2));
             if (I->mode == 2)
             {
                 IND_LAUNCH(I, KI_VECTOR, s, k_vec_comb<<<ge, 256, 0, s>>>(I->ctl.p, ne, I->V.p, I->yv.p, I->w.p));
@@ -601,10 +741,10 @@ int solve_impl(MhdInduction *I, const double *Phi, const double *Ee, const int8_
             }
             else
                 IND_LAUNCH(I, KI_VECTOR, s,
-                           k_vec_update<<<ge, 256, 0, s>>>(I->ctl.p, ne, I->V.p, I->yv.p, I->pd.p, dir, I->x0.p, I->delta.p, I->z.p));
+                           launch_pdl(k_vec_update, ge, 256, 0, s, I->ctl.p, ne, I->V.p, I->yv.p, I->pd.p, dir, I->x0.p, I->delta.p, I->z.p));
             // true residual in FP64 (the outer iterative refinement of the mixed-precision solve)
             apply_plain(I, I->z.p, dtA, I->Ax.p, dte);
-            IND_LAUNCH(I, KI_VECTOR, s, k_vec_resid<<<ge, 256, 0, s>>>(ne, I->b.p, I->Ax.p, dir, I->r.p));
+            IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_vec_resid, ge, 256, 0, s, ne, I->b.p, I->Ax.p, dir, I->r.p));
             dev_dot(I, I->r.p, I->r.p, 1, sc + 1);
             MHD_LAUNCH_CHECK();
             host_read(I, sc + 1, 3);
@@ -612,7 +752,7 @@ int solve_impl(MhdInduction *I, const double *Phi, const double *Ee, const int8_
             total += static_cast<int>(I->pinned[1]);
             I->last_reorth += static_cast<int32_t>(I->pinned[2]);
         }
-        IND_LAUNCH(I, KI_VECTOR, s, k_vec_final<<<ge, 256, 0, s>>>(ne, I->x0.p, I->delta.p, Ee, dir, E, I->corr.p));
+        IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_vec_final, ge, 256, 0, s, ne, I->x0.p, I->delta.p, Ee, dir, E, I->corr.p));
         MHD_LAUNCH_CHECK();
         MHD_CUDA(cudaStreamSynchronize(s));
         if (I->mode == 2) ilu_check(I);

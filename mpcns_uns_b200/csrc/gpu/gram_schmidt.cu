@@ -22,6 +22,9 @@ namespace
 // passes over the basis instead of j + 1: every pass reads w and V_0..V_j once and forms all its dot
 // products together.
 
+constexpr int kGsThreads = 128;
+constexpr int kGsStages = 3; // tiles in flight per block: the one being read and kGsStages - 1 ahead
+
 // Warp reduce-scatter of 32 partial sums: afterwards lane l holds the warp's sum of acc[l] in acc[0].
 __device__ __forceinline__ double warp_reduce_scatter32(double (&acc)[32])
 {
@@ -41,54 +44,18 @@ __device__ __forceinline__ double warp_reduce_scatter32(double (&acc)[32])
     return acc[0];
 }
 
-// The 32 grid-wide sums whose warp sums lane l of every warp holds for index l: block partials, then the
-// last block to finish adds them (in a fixed order: deterministic) into out[0..31] and re-arms the counter.
-// Returns true in that last block (all of its threads), after out is written and visible to them.
-__device__ __forceinline__ bool grid_sum32(double v, double *part, unsigned *counter, double *out)
+// The block's 32 sums (lane l of every warp holds its warp's sum of value l), one row of the partials; gmres.cu's
+// k_cgs_tail adds the rows.
+__device__ __forceinline__ void block_sum32(double v, double *part)
 {
-    __shared__ double sh[8][32];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    sh[wid][lane] = v;
+    __shared__ double sh[kGsThreads / 32][32];
+    sh[threadIdx.x >> 5][threadIdx.x & 31] = v;
     __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[w][threadIdx.x];
-        part[(int64_t)blockIdx.x * 32 + threadIdx.x] = s;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    // every thread of the last block: value v = t % 32 over the blocks b = t / 32 (mod warps), four
-    // accumulators so that the loads overlap; then the warps' sums in warp order
-    {
-        const int k = threadIdx.x >> 5, nk = blockDim.x >> 5;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        unsigned b = k;
-        for (; b + 3u * nk < gridDim.x; b += 4u * nk)
-        {
-            a0 += __ldcg(part + (int64_t)b * 32 + lane);
-            a1 += __ldcg(part + (int64_t)(b + nk) * 32 + lane);
-            a2 += __ldcg(part + (int64_t)(b + 2 * nk) * 32 + lane);
-            a3 += __ldcg(part + (int64_t)(b + 3 * nk) * 32 + lane);
-        }
-        for (; b < gridDim.x; b += nk) a0 += __ldcg(part + (int64_t)b * 32 + lane);
-        sh[k][lane] = (a0 + a1) + (a2 + a3);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[w][threadIdx.x];
-        out[threadIdx.x] = s;
-    }
-    if (threadIdx.x == 0) *counter = 0;
-    __syncthreads();
-    return true;
+    if (threadIdx.x >= 32) return;
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kGsThreads / 32; ++w) s += sh[w][threadIdx.x];
+    part[(int64_t)blockIdx.x * 32 + threadIdx.x] = s;
 }
 
 // The passes are instantiated for every number NV = j + 1 of basis vectors (1..31), so that a thread
@@ -101,18 +68,16 @@ __device__ __forceinline__ bool grid_sum32(double v, double *part, unsigned *cou
 // shared memory (cp.async, kGsStages stages, each thread copying and reading only its own column: no block
 // barrier), so that a thread keeps many loads in flight without holding them in registers.  8-byte copies:
 // the basis vectors start at i * ldv, which need not be 16-byte aligned.
-constexpr int kGsThreads = 128;
-constexpr int kGsStages = 3; // tiles in flight per block: the one being read and kGsStages - 1 ahead
 
-// Pass 1: h_i = V_i . w (i < NV) into H(i, j), and |w|^2 into red[32], over the owned edges.  red holds 96
-// doubles: [0, 31) the re-orthogonalisation dots, [32] |w|^2 before the update, [64, 96) the last pass's sums.
+// Pass 1: the partial sums of h_i = V_i . w (i < NV) and of |w|^2 (value 31) over the owned edges.
 // Dynamic shared memory: kGsStages stages x (NV + 1) vectors x kGsThreads doubles.
 template <int NV>
 __global__ void __launch_bounds__(kGsThreads) k_cgs_dots(Gate gt, const double *__restrict__ w, const double *__restrict__ V, int64_t ldv,
-                                                          int32_t n_owned, double *part, unsigned *counter, double *red, double *H, int mcols)
+                                                          int32_t n_owned, double *part)
 {
+    pdl_begin();
     if (gt.off()) return;
-    constexpr int j = NV - 1, NVEC = NV + 1;
+    constexpr int NVEC = NV + 1;
     extern __shared__ double sm[];
     const int tid = threadIdx.x;
     const int64_t ntiles = (n_owned + kGsThreads - 1) / kGsThreads;
@@ -151,25 +116,21 @@ __global__ void __launch_bounds__(kGsThreads) k_cgs_dots(Gate gt, const double *
     double p[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) p[i] = i < NV ? acc[i] : (i == 31 ? acc[NV] : 0.0);
-    if (!grid_sum32(warp_reduce_scatter32(p), part, counter, red + 64)) return;
-    if (threadIdx.x <= j) H[threadIdx.x * mcols + j] = red[64 + threadIdx.x];
-    if (threadIdx.x == 31) red[32] = red[64 + 31];
+    block_sum32(warp_reduce_scatter32(p), part);
 }
 
 // Pass 2 (and 3): w -= sum_i c_i V_i on every edge, with c = H(:, j) (pass 2) or the re-orthogonalisation
-// dots red[0..j] (pass 3); the next face pass's input zs = w * pd; and over the owned edges the dots
-// s_i = V_i . w and |w|^2 of the result.  Pass 2 (reorth == 0) then decides: if the subtraction cancelled
-// (|w|^2 < |w_before|^2 / 2, red[32] holds |w_before|^2 from pass 1) and the remaining components along
-// the basis are above round-off (|s| > 1e-12 |w|), it leaves s in red[0..j] and raises ctl->reorth; else it
-// stores H(j+1, j) = |w|.  Pass 3 (reorth == 1) runs only when raised: it adds c to H(:, j), stores
-// H(j+1, j) = |w| and lowers the flag.  reverse: the tiles in descending order (the previous pass's tail is
-// in L2).  Dynamic shared memory: kGsStages stages x (NV + 2) vectors (the basis, w, pd) x kGsThreads doubles.
+// dots red[0..j] (pass 3, which runs only when k_cgs_tail raised ctl->reorth); the next face pass's input zs = w * pd;
+// and over the owned edges the partial sums of s_i = V_i . w and |w|^2 of the result.  reverse: the tiles in descending
+// order (the previous pass's tail is in L2).  Dynamic shared memory: kGsStages stages x (NV + 2) vectors (the basis, w,
+// pd) x kGsThreads doubles.
 template <int NV, bool F32>
-__global__ void __launch_bounds__(kGsThreads) k_cgs_update(Gate gt, Ctl *ctl, int reorth, double *__restrict__ w, const double *__restrict__ V,
+__global__ void __launch_bounds__(kGsThreads) k_cgs_update(Gate gt, const Ctl *ctl, int reorth, double *__restrict__ w, const double *__restrict__ V,
                                                             int64_t ldv, int32_t n_all, int32_t n_owned, int reverse, double *part,
-                                                            unsigned *counter, double *red, double *H, int mcols,
-                                                            const double *__restrict__ pd, double *__restrict__ zs, float *__restrict__ zs32)
+                                                            const double *red, const double *H, int mcols, const double *__restrict__ pd,
+                                                            double *__restrict__ zs, float *__restrict__ zs32)
 {
+    pdl_begin();
     if (gt.off() || (reorth && !ctl->reorth)) return;
     constexpr int j = NV - 1, NVEC = NV + 2;
     extern __shared__ double sm[];
@@ -224,55 +185,33 @@ __global__ void __launch_bounds__(kGsThreads) k_cgs_update(Gate gt, Ctl *ctl, in
     double p[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) p[i] = i < NV ? acc[i] : (i == 31 ? acc[NV] : 0.0);
-    // the sums of s and |w|^2 go to red[64..95]; red[32] keeps |w_before|^2 of pass 1
-    const bool last = grid_sum32(warp_reduce_scatter32(p), part, counter, red + 64);
-    if (!last || threadIdx.x != 0) return;
-    const double nn = red[64 + 31];
-    double ss = 0.0;
-    for (int i = 0; i < NV; ++i) ss += red[64 + i] * red[64 + i];
-    if (!reorth && nn < 0.5 * red[32] && ss > 1e-24 * nn)
-    {
-        for (int i = 0; i < NV; ++i) red[i] = red[64 + i];
-        ctl->reorth = 1;
-        ++ctl->n_reorth;
-        return;
-    }
-    if (reorth)
-        for (int i = 0; i < NV; ++i) H[i * mcols + j] += csh[i];
-    H[(j + 1) * mcols + j] = sqrt(nn);
-    ctl->reorth = 0;
+    block_sum32(warp_reduce_scatter32(p), part);
 }
 
 // Launchers of the instances for NV = 1..31, and their grids (resident blocks on every SM)
 constexpr size_t gs_smem(int nvec) { return size_t(kGsStages) * nvec * kGsThreads * sizeof(double); }
 template <int NV> void cgs_step(const CgsArgs &a, const int *grid, cudaStream_t s, int pass)
 {
-    if (pass == 0)
-        k_cgs_dots<NV><<<grid[0], kGsThreads, gs_smem(NV + 1), s>>>(a.gt, a.w, a.V, a.ldv, a.n_owned, a.part, a.counter, a.red, a.H,
-                                                                    a.mcols);
-    else if (a.zs32)
-        k_cgs_update<NV, true><<<grid[1], kGsThreads, gs_smem(NV + 2), s>>>(a.gt, a.ctl, pass - 1, a.w, a.V, a.ldv, a.n_all, a.n_owned,
-                                                                            pass == 1, a.part, a.counter, a.red, a.H, a.mcols, a.pd,
-                                                                            nullptr, a.zs32);
+    if (pass == 0) launch_pdl(k_cgs_dots<NV>, grid[0], kGsThreads, gs_smem(NV + 1), s, a.gt, a.w, a.V, a.ldv, a.n_owned, a.part);
     else
-        k_cgs_update<NV, false><<<grid[1], kGsThreads, gs_smem(NV + 2), s>>>(a.gt, a.ctl, pass - 1, a.w, a.V, a.ldv, a.n_all, a.n_owned,
-                                                                             pass == 1, a.part, a.counter, a.red, a.H, a.mcols, a.pd,
-                                                                             a.zs, nullptr);
+        launch_pdl(a.zs32 ? k_cgs_update<NV, true> : k_cgs_update<NV, false>, grid[1], kGsThreads, gs_smem(NV + 2), s, a.gt, a.ctl, pass - 1,
+                   a.w, a.V, a.ldv, a.n_all, a.n_owned, pass == 1, a.part, a.red, a.H, a.mcols, a.pd, a.zs, a.zs32);
 }
-// the instances' shared memory opted in, and their resident grids (the partials buffer holds kRedBlocks)
+// the instances' shared memory opted in, and their grids: as many blocks as an SM's shared memory holds (with the 3.25 KB
+// that a block's static and reserved part takes), at most 8 (the partials buffer holds kRedBlocks rows).  The grid fixes
+// the order of the sums.
 template <int NV> void cgs_grids(int sms, int *grid)
 {
     const int sd = static_cast<int>(gs_smem(NV + 1)), su = static_cast<int>(gs_smem(NV + 2));
     MHD_CUDA(cudaFuncSetAttribute(k_cgs_dots<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, sd));
     MHD_CUDA(cudaFuncSetAttribute(k_cgs_update<NV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, su));
     MHD_CUDA(cudaFuncSetAttribute(k_cgs_update<NV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, su));
-    int per = 0;
-    MHD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cgs_dots<NV>, kGsThreads, sd));
-    grid[0] = std::max(1, std::min(kRedBlocks, sms * std::max(per, 1)));
-    MHD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cgs_update<NV, false>, kGsThreads, su));
-    int per32 = 0;
-    MHD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per32, k_cgs_update<NV, true>, kGsThreads, su));
-    grid[1] = std::max(1, std::min(kRedBlocks, sms * std::max(std::min(per, per32), 1)));
+    int dev = 0, smem = 0;
+    MHD_CUDA(cudaGetDevice(&dev));
+    MHD_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    auto per = [&](int dyn) { return std::max(1, std::min(8, smem / (dyn + 3328))); };
+    grid[0] = std::min(kRedBlocks, sms * per(sd));
+    grid[1] = std::min(kRedBlocks, sms * per(su));
 }
 using CgsStepFn = void (*)(const CgsArgs &, const int *, cudaStream_t, int);
 using CgsGridFn = void (*)(int, int *);
@@ -289,6 +228,7 @@ const std::array<CgsGridFn, kCgsMax> kCgsGrid = cgs_grid_table(std::make_integer
 
 } // namespace
 
+int cgs_tiles(int32_t n) { return (n + kGsThreads - 1) / kGsThreads; }
 void cgs_launch(int j, const CgsArgs &a, const int *grid, cudaStream_t s, int pass) { kCgsStep[j](a, grid, s, pass); }
 void cgs_grids_for(int k, int sms, int *grid) { kCgsGrid[k](sms, grid); }
 } // namespace mhd

@@ -46,15 +46,16 @@ struct CgsArgs
     const double *V;
     int64_t ldv;
     int32_t n_all, n_owned;
-    double *part, *red, *H;
-    unsigned *counter;
+    double *part, *red, *H; // red: [0, 31) the re-orthogonalisation dots, [32] |w|^2 before the update
     int mcols;
     const double *pd;
     double *zs;
     float *zs32;
 };
-// pass 0: the dots; 1: the update; 2: the gated second update (column j = number of basis vectors - 1)
+// pass 0: the dots; 1: the update; 2: the gated second update (column j = number of basis vectors - 1).  Each leaves one
+// row of 32 partial sums per block; blocks past the last tile (cgs_tiles) leave zeros.
 void cgs_launch(int j, const CgsArgs &a, const int *grid, cudaStream_t s, int pass);
+int cgs_tiles(int32_t n); // tiles of n edges: blocks past them have none
 // the resident grids of column k's passes (2 ints), for an SM count
 void cgs_grids_for(int k, int sms, int *grid);
 
@@ -172,6 +173,7 @@ __device__ __forceinline__ void grid_sum_tail(double v, double *part, unsigned *
 template <class T, bool TRI = false>
 __global__ void k_ind_face(MeshView m, Gate gt, MatIn in, int hall, int resistive, T *__restrict__ phi, T *__restrict__ s2phi)
 {
+    pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nf || gt.off()) return;
     double s = 0;
@@ -218,6 +220,7 @@ __global__ void k_ind_face(MeshView m, Gate gt, MatIn in, int hall, int resistiv
 template <class T, bool TET = false>
 __global__ void k_ind_bcell(MeshView m, Gate gt, const T *__restrict__ recon, const T *__restrict__ phi, T *__restrict__ b)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc || gt.off()) return;
     T bx = 0, by = 0, bz = 0;
@@ -238,6 +241,7 @@ __global__ void k_ind_hall32(MeshView m, Gate gt, const float4 *__restrict__ slo
                              const float *__restrict__ alpha, const float *__restrict__ B0, const float *__restrict__ vinv,
                              float *__restrict__ g)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.no_cells || gt.off()) return;
     const float a = alpha[c];
@@ -282,6 +286,7 @@ __global__ void k_ind_hall32(MeshView m, Gate gt, const float4 *__restrict__ slo
 template <class T, int MAXK>
 __global__ void __launch_bounds__(256) k_ind_edge(MeshView m, EdgeArgs<T> a)
 {
+    pdl_begin();
     if (a.gt.off()) return;
     const int32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     double contrib = 0.0;
