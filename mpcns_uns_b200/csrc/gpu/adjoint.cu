@@ -1427,6 +1427,7 @@ static const char *const kFnKernelNames[FN_COUNT] = {"forward_steps", "record_st
 
 struct MhdFn
 {
+    Hold<MhdState> hold; // first: released last
     MhdState *st = nullptr;
     MhdFnParams prm{};
     int nsp = 0;
@@ -1853,6 +1854,7 @@ int mhd_gpu_fn_create(MhdState *st, const MhdFnParams *p, const double *eta, con
         MHD_REQUIRE(p->n_steps >= 1 && p->checkpoint_every >= 1 && p->dt > 0, "need n_steps >= 1, checkpoint_every >= 1, dt > 0");
         fn = new MhdFn;
         fn->st = st;
+        fn->hold.take(st);
         fn->prm = *p;
         fn->nsp = st->nsp;
         for (int a = 0; a < 3; ++a) fn->u_inf[a] = fn->u_create[a] = st->prm.u_inf[a];

@@ -304,8 +304,32 @@ template <int N> struct EventProfiler
 };
 } // namespace mhd
 
+namespace mhd
+{
+// A handle that others are built on lives until its destroy call and the last of those others are gone, in any order
+// (a host's garbage collector may finalise a mesh before the handles made on it).
+template <class T> void drop_ref(T *t)
+{
+    if (t && t->refs.fetch_sub(1) == 1) delete t;
+}
+template <class T> struct Hold
+{
+    T *p = nullptr;
+    Hold() = default;
+    Hold(const Hold &) = delete;
+    Hold &operator=(const Hold &) = delete;
+    void take(T *t)
+    {
+        t->refs.fetch_add(1);
+        p = t;
+    }
+    ~Hold() { drop_ref(p); }
+};
+} // namespace mhd
+
 struct MhdMesh
 {
+    std::atomic<int> refs{1};
     mhd::MeshView v{};
     cudaStream_t stream = nullptr;
     bool own_stream = false;

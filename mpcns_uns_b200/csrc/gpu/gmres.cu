@@ -793,6 +793,7 @@ int mhd_gpu_induction_create(MhdMesh *mesh, const MhdInductionParams *p, const d
         cudaStream_t s = mesh->stream;
         I = new MhdInduction;
         I->mesh = mesh;
+        I->hold.take(mesh);
         I->p = *p;
         I->p.restart = std::max(2, p->restart); // restart_(std::max(2, cfg.ind_restart)) of the constructor
         I->hall = p->hall && p->hall_coef > 0;

@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(256) k_ind_edge(MeshView m, EdgeArgs<T> a)
 
 struct MhdInduction
 {
+    mhd::Hold<MhdMesh> hold; // first: released last
     MhdMesh *mesh = nullptr;
     MhdInductionParams p{};
     bool resistive = false, hall = false, mixed = false, have_corr = false;

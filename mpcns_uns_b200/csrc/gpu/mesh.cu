@@ -451,7 +451,7 @@ int mhd_gpu_mesh_destroy(MhdMesh *mesh)
     return guarded([&] {
         if (!mesh) return;
         if (mesh->stream) cudaStreamSynchronize(mesh->stream);
-        delete mesh;
+        drop_ref(mesh);
     });
 }
 

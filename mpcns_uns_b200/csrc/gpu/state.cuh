@@ -38,6 +38,8 @@ struct MixedTables
 
 struct MhdState
 {
+    std::atomic<int> refs{1};
+    mhd::Hold<MhdMesh> hold; // first: released last
     MhdMesh *mesh = nullptr;
     MhdStepParams prm{};
     mhd::FluidParams fp{};

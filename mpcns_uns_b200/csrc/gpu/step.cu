@@ -511,6 +511,7 @@ int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *p, MhdState **out)
         MHD_REQUIRE(!p->ambipolar || mesh->v.e_nodes, "the ambipolar EMF needs the mesh's edge_nodes");
         st = new MhdState;
         st->mesh = mesh;
+        st->hold.take(mesh);
         st->prm = *p;
         st->nsp = p->n_species;
         st->group = std::min(kGroup, st->nsp);
@@ -603,7 +604,7 @@ int mhd_gpu_state_destroy(MhdState *st)
     return guarded([&] {
         if (!st) return;
         cudaStreamSynchronize(st->mesh->stream);
-        delete st;
+        drop_ref(st);
     });
 }
 
