@@ -167,6 +167,7 @@ template <int NF, int NS, int SI, bool LOG, bool GRAD, bool FACE>
 __global__ void __launch_bounds__(160, NF == 4 ? 6 : 5) k_limited_slots(MeshView m, FluidParams p, SField<const double> W,
                                                                               SField<double> G, double *__restrict__ FV)
 {
+    pdl_begin();
     constexpr int ROWS = 6 * NF + 6; // w d (3 per slot), dx (3 per slot), inverse (6)
     __shared__ double geo[ROWS][32];
     __shared__ uint32_t pos[2][NS][NF]; // per face slot the cells whose density (0) / pressure (1) there is positive
@@ -355,10 +356,10 @@ void launch_slots(const MeshView &m, FluidParams p, SField<const double> W, SFie
     {
         const bool pair = nsp - s0 > 1;
         if (W.si == 1)
-            (pair ? k_limited_slots<NF, 2, 1, LOG, GRAD, FACE> : k_limited_slots<NF, 1, 1, LOG, GRAD, FACE>)<<<grid, block, 0, s>>>(m, p, W,
-                                                                                                                                G, FV);
+            launch_pdl(pair ? k_limited_slots<NF, 2, 1, LOG, GRAD, FACE> : k_limited_slots<NF, 1, 1, LOG, GRAD, FACE>, grid, block, 0, s, m, p,
+                       W, G, FV);
         else if constexpr (!FACE && !LOG) // the reference's layout: one species a call
-            k_limited_slots<NF, 1, 5, false, GRAD, false><<<grid, block, 0, s>>>(m, p, W, G, FV);
+            launch_pdl(k_limited_slots<NF, 1, 5, false, GRAD, false>, grid, block, 0, s, m, p, W, G, FV);
         // the next pair's species become 0 and 1
         W.p += 2 * W.ss;
         if (GRAD) G.p += 2 * G.ss;
@@ -457,6 +458,7 @@ __global__ void __launch_bounds__(128) k_face_flux(MeshView m, FluidParams p, SF
 __global__ void __launch_bounds__(128) k_face_flux_fv(MeshView m, FluidParams p, int64_t nnz, const double *__restrict__ FV,
                                                       double *__restrict__ F)
 {
+    pdl_begin();
     const int s = blockIdx.x % p.nsp;
     const int32_t f = (blockIdx.x / p.nsp) * blockDim.x + threadIdx.x;
     if (f >= m.nf) return;
@@ -549,7 +551,7 @@ void launch_face_values(const MeshView &m, const FluidParams &p, SField<const do
 void launch_face_flux_fv(const MeshView &m, const FluidParams &p, const double *FV, double *F, cudaStream_t s)
 {
     if (!m.nf) return;
-    k_face_flux_fv<<<grid_for(m.nf, 128) * p.nsp, 128, 0, s>>>(m, p, (int64_t)m.faces_per_cell * m.nc, FV, F);
+    launch_pdl(k_face_flux_fv, grid_for(m.nf, 128) * p.nsp, 128, 0, s, m, p, (int64_t)m.faces_per_cell * m.nc, FV, F);
     MHD_LAUNCH_CHECK();
 }
 

@@ -28,6 +28,7 @@ __global__ void k_face_candidate(MeshView m, const double *__restrict__ u, const
                                  const double *__restrict__ phi_tot, const double *__restrict__ phi_add, double *__restrict__ Ef,
                                  double *__restrict__ pa, uint32_t *__restrict__ sw)
 {
+    pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nf) return;
     const double A = m.face_area_mag[f];
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(128, GEO ? 6 : 4) k_edge_emf_assign(MeshView m
                                                                     uint32_t *__restrict__ sw, const double *__restrict__ geo,
                                                                     const double *__restrict__ pa)
 {
+    pdl_begin();
     __shared__ double su[GEO ? 3 * kGeoCells * 128 : 1];
     const int32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= m.ne) return;
@@ -379,7 +381,7 @@ void launch_face_candidate(const MeshView &m, const double *u, const double *Bt,
                            const double *phi_add, double *Ef, cudaStream_t s, double *pa, uint32_t *sw)
 {
     if (!m.nf) return;
-    k_face_candidate<<<grid_for(m.nf, 128), 128, 0, s>>>(m, u, Bt, Bi, phi_tot, phi_add, Ef, pa, sw);
+    launch_pdl(k_face_candidate, grid_for(m.nf, 128), 128, 0, s, m, u, Bt, Bi, phi_tot, phi_add, Ef, pa, sw);
     MHD_LAUNCH_CHECK();
 }
 
@@ -389,16 +391,11 @@ void launch_edge_emf_assign(const MeshView &m, const double *Ef, const double *u
 {
     if (!m.ne) return;
     const int g = grid_for(m.ne, 128);
-    if (geo && pa && m.max_edge_cells <= kGeoCells && m.max_valence <= kGeoSlots)
-        (sw ? k_edge_emf_assign<8, true, true> : k_edge_emf_assign<8, false, true>)<<<g, 128, 0, s>>>(m, Ef, u, phi_ind, cuct, E_inf, mres,
-                                                                                                      amb, E, sw, geo, pa);
-    else if (m.max_valence <= 8)
-        (sw ? k_edge_emf_assign<8, true, false> : k_edge_emf_assign<8, false, false>)<<<g, 128, 0, s>>>(m, Ef, u, phi_ind, cuct, E_inf, mres,
-                                                                                                        amb, E, sw, nullptr, nullptr);
-    else
-        (sw ? k_edge_emf_assign<kMaxValence, true, false>
-            : k_edge_emf_assign<kMaxValence, false, false>)<<<g, 128, 0, s>>>(m, Ef, u, phi_ind, cuct, E_inf, mres, amb, E, sw, nullptr,
-                                                                               nullptr);
+    const bool table = geo && pa && m.max_edge_cells <= kGeoCells && m.max_valence <= kGeoSlots;
+    auto k = table ? (sw ? k_edge_emf_assign<8, true, true> : k_edge_emf_assign<8, false, true>)
+             : m.max_valence <= 8 ? (sw ? k_edge_emf_assign<8, true, false> : k_edge_emf_assign<8, false, false>)
+                                  : (sw ? k_edge_emf_assign<kMaxValence, true, false> : k_edge_emf_assign<kMaxValence, false, false>);
+    launch_pdl(k, g, 128, 0, s, m, Ef, u, phi_ind, cuct, E_inf, mres, amb, E, sw, table ? geo : nullptr, table ? pa : nullptr);
     MHD_LAUNCH_CHECK();
 }
 
@@ -513,6 +510,7 @@ __global__ void __launch_bounds__(1024) k_div_b_final(const DivPart *__restrict_
 // mhd::cell_current (Common/induction/Current.cpp:9-31)
 __global__ void k_cell_current(MeshView m, const double *__restrict__ B, double *__restrict__ J)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     if (c >= m.no_cells)
@@ -594,7 +592,7 @@ double *noalloc_scratch()
 void launch_cell_current(const MeshView &m, const double *B, double *J, cudaStream_t s)
 {
     if (!m.nc) return;
-    k_cell_current<<<grid_for(m.nc, 128), 128, 0, s>>>(m, B, J);
+    launch_pdl(k_cell_current, grid_for(m.nc, 128), 128, 0, s, m, B, J);
     MHD_LAUNCH_CHECK();
 }
 
@@ -602,7 +600,7 @@ void ideal_emf_enqueue(const MeshView &m, const double *u, const double *Bt, con
                        const double *phi_ind, double cuct, double *face3, double *E, cudaStream_t s)
 {
     if (!m.nf) return;
-    k_face_candidate<<<grid_for(m.nf, 128), 128, 0, s>>>(m, u, Bt, Bi, phi_tot, nullptr, face3, nullptr, nullptr);
+    launch_pdl(k_face_candidate, grid_for(m.nf, 128), 128, 0, s, m, u, Bt, Bi, phi_tot, nullptr, face3, nullptr, nullptr);
     if (m.no_edges)
     {
         if (m.max_valence <= 8)

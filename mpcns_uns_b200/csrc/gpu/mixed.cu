@@ -272,65 +272,132 @@ __device__ __forceinline__ void rusanov32(const F5 &L, const F5 &R, float3 n, fl
     F[4] = 0.5f * (unL * (EL + L.p) + unR * (ER + R.p)) - 0.5f * s * (ER - EL);
 }
 
-// per-cell primitives (FP32, 32 bytes per species) and the charge-weighted velocity u+ of cell c
+// per-cell primitives (FP32, 32 bytes per species) and the charge-weighted velocity u+ of cell c.  NSP: the number of
+// species, whose primitives then stay in w (0: any number, re-read where they are needed); store: write W and up.
+template <int NSP>
 __device__ __forceinline__ void mx_prims(const MxParams &p, int64_t n, const double *__restrict__ U, float4 *__restrict__ W,
-                                         float4 *__restrict__ up, int32_t c, bool fluid)
+                                         float4 *__restrict__ up, int32_t c, bool fluid, F5 (&w5)[NSP ? NSP : 1], bool store = true)
 {
+    const int nsp = NSP ? NSP : p.nsp;
     float ne = 0.f;
     double pe = 0.0;
-    for (int s = 0; s < p.nsp; ++s)
+#pragma unroll
+    for (int s = 0; s < nsp; ++s)
     {
         const double *Us = U + (int64_t)s * 5 * n;
         const double r = fmax(Us[c], p.rho_floor_d);
         const double ir = 1.0 / r;
         const double u = Us[n + c] * ir, v = Us[2 * n + c] * ir, w = Us[3 * n + c] * ir;
         const double pr = fmax((p.gamma_d - 1.0) * (Us[4 * n + c] - 0.5 * r * (u * u + v * v + w * w)), p.p_floor_d);
-        float4 *Wc = W + 2 * ((int64_t)s * n + c);
-        Wc[0] = make_float4(static_cast<float>(r), static_cast<float>(u), static_cast<float>(v), static_cast<float>(w));
-        Wc[1] = make_float4(static_cast<float>(pr), 0.f, 0.f, 0.f);
-        ne += static_cast<float>(r) / p.mass[s] * p.M_ref;
+        const F5 q{static_cast<float>(r), static_cast<float>(u), static_cast<float>(v), static_cast<float>(w), static_cast<float>(pr)};
+        if (NSP) w5[s] = q;
+        if (!NSP || store)
+        {
+            float4 *Wc = W + 2 * ((int64_t)s * n + c);
+            Wc[0] = make_float4(q.rho, q.u, q.v, q.w);
+            Wc[1] = make_float4(q.p, 0.f, 0.f, 0.f);
+        }
+        ne += q.rho / p.mass[s] * p.M_ref;
         if (s < 2) pe += pr;
     }
     // with the ambipolar terms on, the FP64 electron pressure p_H + p_Na rides in the padding of species 0's
     // pressure slot (.z = high word, .w = low word): the gradients of p_e are differences of nearly equal
     // values that FP32 pressures would not resolve
-    if (p.ambi)
-        W[2 * (int64_t)c + 1] = make_float4(W[2 * (int64_t)c + 1].x, 0.f, __int_as_float(__double2hiint(pe)),
+    if (p.ambi && store)
+        W[2 * (int64_t)c + 1] = make_float4(NSP ? w5[0].p : W[2 * (int64_t)c + 1].x, 0.f, __int_as_float(__double2hiint(pe)),
                                             __int_as_float(__double2loint(pe)));
     float u3[3] = {0.f, 0.f, 0.f};
     if (fluid)
-        for (int s = 0; s < p.nsp; ++s)
+#pragma unroll
+        for (int s = 0; s < nsp; ++s)
         {
-            // number density and velocity re-read from the primitives this thread has just written
-            const float4 wv = W[2 * ((int64_t)s * n + c)];
+            const float4 wv = NSP ? make_float4(w5[s].rho, w5[s].u, w5[s].v, w5[s].w) : W[2 * ((int64_t)s * n + c)];
             const float chi = ne > 1e-30f ? (wv.x / p.mass[s] * p.M_ref) / ne : (s == 0 ? 1.f : 0.f);
             u3[0] += chi * wv.y;
             u3[1] += chi * wv.z;
             u3[2] += chi * wv.w;
         }
-    up[c] = make_float4(u3[0], u3[1], u3[2], 0.f);
+    if (store) up[c] = make_float4(u3[0], u3[1], u3[2], 0.f);
 }
 
-// primitives (FP32), cell field fit, total field, charge-weighted velocity
+// The CFL step of one fluid cell (step.cu's cell_dt, FP32)
+template <int NSP>
+__device__ __forceinline__ float mx_cell_dt(const MV &m, const MxParams &p, float cfl, float inver_MA2, float rho_floor_dt,
+                                            const float4 *__restrict__ W, const F5 (&w5)[NSP ? NSP : 1], float3 b, int4 fi, int32_t c)
+{
+    const int nsp = NSP ? NSP : p.nsp;
+    const int64_t n = m.nc;
+    const float B2 = fdot(b, b);
+    float rs = 0.f;
+#pragma unroll
+    for (int s = 0; s < nsp; ++s) rs += NSP ? w5[s].rho : W[2 * ((int64_t)s * n + c)].x;
+    const float rho_tot = fmaxf(rs, rho_floor_dt);
+    const float4 fn4[4] = {m.fn[fi.x], m.fn[fi.y], m.fn[fi.z], m.fn[fi.w]};
+    const float vol = 1.f / m.vol_inv[c];
+    float dt = CUDART_INF_F;
+#pragma unroll
+    for (int s = 0; s < nsp; ++s)
+    {
+        const float4 wa = NSP ? make_float4(w5[s].rho, w5[s].u, w5[s].v, w5[s].w) : W[2 * ((int64_t)s * n + c)];
+        const float rho = wa.x, u = wa.y, v = wa.z, w = wa.w, pr = NSP ? w5[s].p : W[2 * ((int64_t)s * n + c) + 1].x;
+        const float cs2 = p.gamma * pr / fmaxf(rho, 1e-30f);
+        const float vA2 = inver_MA2 * B2 / rho_tot;
+        float denom = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const float3 nr = f3(fn4[j]);
+            const float bn = fdot(b, nr);
+            const float vAn2 = inver_MA2 * bn * bn / rho_tot;
+            const float term = cs2 + vA2;
+            const float disc = __fmaf_rn(-(4.f * cs2), vAn2, term * term); // rounded alike in every instance
+            const float cf = sqrtf(0.5f * (term + sqrtf(fmaxf(0.f, disc))));
+            denom += (fabsf(u * nr.x + v * nr.y + w * nr.z) + cf) * fn4[j].w;
+        }
+        if (denom > 0.f) dt = fminf(dt, cfl * vol / denom);
+    }
+    return dt;
+}
+
+struct MxCfl
+{
+    float cfl, inver_MA2, rho_floor_dt;
+    int turned; // the opening gyration follows: it writes W and up of the owned fluid cells itself
+    CflOut out;
+};
+
+// primitives (FP32), cell field fit, total field, charge-weighted velocity; with CFL the step size from the values at
+// hand, finished by the last block
+template <int NSP, bool CFL>
 __global__ void __launch_bounds__(128) k_mx_prepare(MV m, MxParams p, const double *__restrict__ U, const double *__restrict__ phi,
                                                      const float4 *__restrict__ badd, float4 *__restrict__ W, float4 *__restrict__ up,
-                                                     float4 *__restrict__ bt, float4 *__restrict__ bi)
+                                                     float4 *__restrict__ bt, float4 *__restrict__ bi, MxCfl cfl)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.nc) return;
     const int64_t n = m.nc;
-    mx_prims(p, n, U, W, up, c, m.material[c] == 0);
-    const int4 fi = *reinterpret_cast<const int4 *>(m.c2f_idx + 4 * (int64_t)c);
-    const float ph[4] = {static_cast<float>(phi[fi.x]), static_cast<float>(phi[fi.y]), static_cast<float>(phi[fi.z]),
-                         static_cast<float>(phi[fi.w])};
-    float b[3] = {0.f, 0.f, 0.f};
+    float dt = CUDART_INF_F;
+    if (c < m.nc)
+    {
+        F5 w5[NSP ? NSP : 1];
+        const int mat = m.material[c];
+        mx_prims<NSP>(p, n, U, W, up, c, mat == 0, w5, !CFL || !cfl.turned || c >= m.no_cells || mat == 1);
+        const int4 fi = *reinterpret_cast<const int4 *>(m.c2f_idx + 4 * (int64_t)c);
+        const float ph[4] = {static_cast<float>(phi[fi.x]), static_cast<float>(phi[fi.y]), static_cast<float>(phi[fi.z]),
+                             static_cast<float>(phi[fi.w])};
+        float b[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) b[a] += m.recon[(3 * j + a) * n + c] * ph[j];
-    const float4 ba = badd[c];
-    bi[c] = make_float4(b[0], b[1], b[2], 0.f);
-    bt[c] = make_float4(b[0] + ba.x, b[1] + ba.y, b[2] + ba.z, 0.f);
+            for (int a = 0; a < 3; ++a) b[a] += m.recon[(3 * j + a) * n + c] * ph[j];
+        const float4 ba = badd[c];
+        const float3 t = make_float3(b[0] + ba.x, b[1] + ba.y, b[2] + ba.z);
+        bi[c] = make_float4(b[0], b[1], b[2], 0.f);
+        bt[c] = make_float4(t.x, t.y, t.z, 0.f);
+        if (CFL && c < m.no_cells && mat == 0)
+            dt = mx_cell_dt<NSP>(m, p, cfl.cfl, cfl.inver_MA2, cfl.rho_floor_dt, W, w5, t, fi, c);
+    }
+    if constexpr (CFL) cfl_reduce(cfl.out, dt > 0.f ? static_cast<double>(dt) : CUDART_INF, !(dt > 0.f));
 }
 
 // The opening half-step gyration (mercury::gyrate, FP64 on the FP64 state, FP32 total field) with the
@@ -340,6 +407,7 @@ __global__ void __launch_bounds__(128) k_mx_gyrate(MV m, MxParams p, SrcParams s
                                                    const double *__restrict__ dtp, double scale, double *__restrict__ U,
                                                    float4 *__restrict__ W, float4 *__restrict__ up)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.no_cells || m.material[c] == 1) return;
     const int64_t n = m.nc;
@@ -355,59 +423,8 @@ __global__ void __launch_bounds__(128) k_mx_gyrate(MV m, MxParams p, SrcParams s
         U[q * n + c] = uh[q];
         U[(5 + q) * n + c] = un[q];
     }
-    mx_prims(p, n, U, W, up, c, m.material[c] == 0);
-}
-
-__global__ void __launch_bounds__(128) k_mx_cfl(MV m, MxParams p, float cfl, float inver_MA2, float rho_floor_dt,
-                                                 const float4 *__restrict__ W, const float4 *__restrict__ bt,
-                                                 unsigned long long *__restrict__ dt_bits, int *__restrict__ flag)
-{
-    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t n = m.nc;
-    float dt = CUDART_INF_F;
-    if (c < m.no_cells && m.material[c] == 0)
-    {
-        const float3 b = f3(bt[c]);
-        const float B2 = fdot(b, b);
-        float rs = 0.f;
-        for (int s = 0; s < p.nsp; ++s) rs += W[2 * ((int64_t)s * n + c)].x;
-        const float rho_tot = fmaxf(rs, rho_floor_dt);
-        const int4 fi = *reinterpret_cast<const int4 *>(m.c2f_idx + 4 * (int64_t)c);
-        const float4 fn4[4] = {m.fn[fi.x], m.fn[fi.y], m.fn[fi.z], m.fn[fi.w]};
-        const float vol = 1.f / m.vol_inv[c];
-        for (int s = 0; s < p.nsp; ++s)
-        {
-            const float4 wa = W[2 * ((int64_t)s * n + c)];
-            const float rho = wa.x, u = wa.y, v = wa.z, w = wa.w, pr = W[2 * ((int64_t)s * n + c) + 1].x;
-            const float cs2 = p.gamma * pr / fmaxf(rho, 1e-30f);
-            const float vA2 = inver_MA2 * B2 / rho_tot;
-            float denom = 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-            {
-                const float3 nr = f3(fn4[j]);
-                const float bn = fdot(b, nr);
-                const float vAn2 = inver_MA2 * bn * bn / rho_tot;
-                const float term = cs2 + vA2;
-                const float cf = sqrtf(0.5f * (term + sqrtf(fmaxf(0.f, term * term - 4.f * cs2 * vAn2))));
-                denom += (fabsf(u * nr.x + v * nr.y + w * nr.z) + cf) * fn4[j].w;
-            }
-            if (denom > 0.f) dt = fminf(dt, cfl * vol / denom);
-        }
-        if (!(dt > 0.f)) atomicOr(flag, 1);
-    }
-    __shared__ float sh[32];
-    float v = dt > 0.f ? dt : CUDART_INF_F;
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : CUDART_INF_F;
-        for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (threadIdx.x == 0 && v < CUDART_INF_F)
-            atomicMin(dt_bits, static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(v))));
-    }
+    F5 w5[2];
+    mx_prims<2>(p, n, U, W, up, c, m.material[c] == 0, w5);
 }
 
 // limited face values (see below) of cell c for species s0 + g of a group of ng: FV[(q*n + c)*ng + g] holds
@@ -702,6 +719,7 @@ __global__ void __launch_bounds__(128) k_mx_face_cand(MV m, const float4 *__rest
                                                       const double *__restrict__ phi_add, float4 *__restrict__ Ef,
                                                       float4 *__restrict__ G, const float4 *__restrict__ W, float4 *__restrict__ D)
 {
+    pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nf) return;
     const float4 nf4 = m.fn[f];
@@ -759,6 +777,7 @@ __global__ void __launch_bounds__(128) k_mx_face_cand(MV m, const float4 *__rest
 __global__ void __launch_bounds__(128, 8) k_mx_edge(MV m, const float4 *__restrict__ Ef, const float4 *__restrict__ up,
                                                     float cuct, float3 E_inf, float *__restrict__ E)
 {
+    pdl_begin();
     const int32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= m.ne) return;
     float val = 0.f;
@@ -840,6 +859,7 @@ __global__ void __launch_bounds__(256) k_mx_ct(int32_t nf, const int4 *__restric
                                                const double *__restrict__ phis, double *__restrict__ phio, const double *__restrict__ dtp,
                                                int stage2)
 {
+    pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
     const int4 r = fe[f];
@@ -865,20 +885,6 @@ __global__ void k_mx_face_edges(MeshView m, int4 *fe)
     fe[f] = make_int4(m.f2e_idx[k0], m.f2e_idx[k0 + 1], m.f2e_idx[k0 + 2], w);
 }
 
-__global__ void k_mx_cfl_init(unsigned long long *dt_bits, int *flag)
-{
-    *dt_bits = static_cast<unsigned long long>(__double_as_longlong(CUDART_INF));
-    *flag = 0;
-}
-
-__global__ void k_mx_cfl_final(const unsigned long long *dt_bits, double dt_max, double *dt, int *flag)
-{
-    double g = __longlong_as_double(static_cast<long long>(*dt_bits));
-    g = fmin(g, dt_max);
-    if (!isfinite(g) || g <= 0) atomicOr(flag, 1);
-    *dt = g;
-}
-
 // Face values and fluxes: the species of a group run as adjacent threads (thread t: cell or face t / ng,
 // species t % ng).  The two threads of a cell read the same stencil tables (one load serves both), write
 // the adjacent float4s of its face values, and the two threads of a face read adjacent face values and
@@ -888,6 +894,7 @@ __global__ void k_mx_cfl_final(const unsigned long long *dt_bits, double dt_max,
 __global__ void __launch_bounds__(128) k_mx_grad(MV m, MxParams p, int s0, int ng, const float4 *__restrict__ W,
                                                  float4 *__restrict__ FV)
 {
+    pdl_begin();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t c = ng == 2 ? t >> 1 : t;
     if (c >= m.nc) return;
@@ -896,6 +903,7 @@ __global__ void __launch_bounds__(128) k_mx_grad(MV m, MxParams p, int s0, int n
 
 __global__ void __launch_bounds__(128) k_mx_flux(MV m, MxParams p, int s0, int ng, const float *__restrict__ FV, float *__restrict__ F)
 {
+    pdl_begin();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t f = ng == 2 ? t >> 1 : t;
     if (f >= m.nf) return;
@@ -912,6 +920,7 @@ __global__ void __launch_bounds__(128) k_mx_update(MV m, MxParams p, int s0, int
                                                    const float4 *__restrict__ bt, SrcParams sp, int gyr, const float4 *__restrict__ D,
                                                    const double *__restrict__ photo, const double *__restrict__ vst)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int64_t n = m.nc;
@@ -1020,6 +1029,7 @@ __global__ void k_mx_node_pressure(int32_t nn, const int32_t *__restrict__ n2c_p
                                    const double *__restrict__ vol, const float4 *__restrict__ W, double *__restrict__ pn,
                                    int8_t *__restrict__ pok)
 {
+    pdl_begin();
     const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nn) return;
     double s = 0, w = 0;
@@ -1037,6 +1047,7 @@ __global__ void k_mx_node_pressure(int32_t nn, const int32_t *__restrict__ n2c_p
 __global__ void k_mx_ambipolar(MV m, MxParams p, const float4 *__restrict__ W, const double *__restrict__ ecw, const int32_t *__restrict__ en,
                                const double *__restrict__ pn, const int8_t *__restrict__ pok, float coef, float *__restrict__ E)
 {
+    pdl_begin();
     const int32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= m.no_edges || m.edge_mode[e] != 0) return;
     float rH = 0.f, rN = 0.f, wsum = 0.f;
@@ -1129,7 +1140,7 @@ void mixed_badd(MhdState *st)
     MHD_LAUNCH_CHECK();
 }
 
-void mixed_prepare(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max)
+void mixed_prepare(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max, bool turned)
 {
     MhdMesh *mesh = st->mesh;
     const MV m = make_view(mesh->v, st->mt);
@@ -1137,31 +1148,26 @@ void mixed_prepare(MhdState *st, const double *Us, const double *phis, bool cfl,
     Profiler &P = st->prof;
     const MxParams p = mx_params(st);
     const int gc = grid_for(m.nc, 128);
-    if (!m.nc) return;
+    if (!m.nc)
+    {
+        if (cfl) cfl_empty(st, dt_max);
+        return;
+    }
     float4 *W4 = reinterpret_cast<float4 *>(st->W32.p);
     P.begin(KP_PREPARE, s);
-    k_mx_prepare<<<gc, 128, 0, s>>>(m, p, Us, phis, st->badd32.p, W4, st->up32.p, st->bt32.p, st->bi32.p);
-    MHD_LAUNCH_CHECK();
+    const MxCfl mc{static_cast<float>(st->prm.cfl), static_cast<float>(st->prm.inver_MA2), static_cast<float>(st->prm.rho_floor_dt),
+                   turned ? 1 : 0, cfl_out(st, dt_max)};
+    auto k = st->nsp == 2 ? (cfl ? k_mx_prepare<2, true> : k_mx_prepare<2, false>) : (cfl ? k_mx_prepare<0, true> : k_mx_prepare<0, false>);
+    launch_pdl(k, gc, 128, 0, s, m, p, Us, phis, st->badd32.p, W4, st->up32.p, st->bt32.p, st->bi32.p, mc);
     ++st->launches;
     P.end(KP_PREPARE, s);
-    if (cfl)
-    {
-        P.begin(KP_CFL, s);
-        k_mx_cfl_init<<<1, 1, 0, s>>>(st->dt_bits.p, st->flag.p);
-        k_mx_cfl<<<gc, 128, 0, s>>>(m, p, static_cast<float>(st->prm.cfl), static_cast<float>(st->prm.inver_MA2),
-                                    static_cast<float>(st->prm.rho_floor_dt), W4, st->bt32.p, st->dt_bits.p, st->flag.p);
-        k_mx_cfl_final<<<1, 1, 0, s>>>(st->dt_bits.p, dt_max, st->scal.p, st->flag.p);
-        MHD_LAUNCH_CHECK();
-        P.end(KP_CFL, s);
-        st->launches += 3;
-    }
 }
 
 void mixed_gyrate_open(MhdState *st)
 {
     const MV m = make_view(st->mesh->v, st->mt);
     if (!m.no_cells) return;
-    k_mx_gyrate<<<grid_for(m.no_cells, 128), 128, 0, st->mesh->stream>>>(m, mx_params(st), st->src, st->bt32.p, st->scal.p, 0.5,
+    launch_pdl(k_mx_gyrate, grid_for(m.no_cells, 128), 128, 0, st->mesh->stream, m, mx_params(st), st->src, st->bt32.p, st->scal.p, 0.5,
                                                                             st->U0.p, reinterpret_cast<float4 *>(st->W32.p), st->up32.p);
     MHD_LAUNCH_CHECK();
     ++st->launches;
@@ -1177,13 +1183,17 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
     Profiler &P = st->prof;
     const MxParams p = mx_params(st);
     const int gc = grid_for(m.nc, 128), gf = grid_for(m.nf, 128), ge = grid_for(m.ne, 128);
-    if (!m.nc) return;
+    if (!m.nc)
+    {
+        if (cfl) cfl_empty(st, dt_max);
+        return;
+    }
     float4 *W4 = reinterpret_cast<float4 *>(st->W32.p);
-    if (!prepared) mixed_prepare(st, Us, phis, cfl, dt_max);
+    if (!prepared) mixed_prepare(st, Us, phis, cfl, dt_max, false);
     // face EMF candidates first: with the J x B force on, this pass also leaves the face terms of the
     // cell current that the update gathers
     P.begin(KP_FACE_CAND, s);
-    k_mx_face_cand<<<gf, 128, 0, s>>>(m, st->up32.p, st->bt32.p, st->bi32.p, phis, st->phi_add.p, st->Ef32.p,
+    launch_pdl(k_mx_face_cand, gf, 128, 0, s, m, st->up32.p, st->bt32.p, st->bi32.p, phis, st->phi_add.p, st->Ef32.p,
                                       st->src.on ? st->g32.p : nullptr, W4, st->src.ambi ? st->d32.p : nullptr);
     MHD_LAUNCH_CHECK();
     P.end(KP_FACE_CAND, s);
@@ -1191,18 +1201,18 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
     {
         const int ng = std::min(st->group, st->nsp - s0);
         P.begin(KP_GRAD, s);
-        k_mx_grad<<<grid_for(static_cast<int64_t>(m.nc) * ng, 128), 128, 0, s>>>(m, p, s0, ng, W4,
+        launch_pdl(k_mx_grad, grid_for(static_cast<int64_t>(m.nc) * ng, 128), 128, 0, s, m, p, s0, ng, W4,
                                                                                    reinterpret_cast<float4 *>(st->grad32.p));
         MHD_LAUNCH_CHECK();
         P.end(KP_GRAD, s);
         P.begin(KP_FLUX, s);
-        k_mx_flux<<<grid_for(static_cast<int64_t>(m.nf) * ng, 128), 128, 0, s>>>(m, p, s0, ng, st->grad32.p, st->F32.p);
+        launch_pdl(k_mx_flux, grid_for(static_cast<int64_t>(m.nf) * ng, 128), 128, 0, s, m, p, s0, ng, st->grad32.p, st->F32.p);
         MHD_LAUNCH_CHECK();
         P.end(KP_FLUX, s);
         P.begin(KP_UPDATE, s);
         // the instance with the closing gyration fused carries its registers; the other stages use the lean one
         auto upd = gyrate_close && s0 == 0 ? k_mx_update<true> : k_mx_update<false>;
-        upd<<<gc, 128, 0, s>>>(m, p, s0, ng, st->F32.p, Us, Uo, st->scal.p, stage2 ? 1 : 0, st->g32.p, st->bt32.p, st->src,
+        launch_pdl(upd, gc, 128, 0, s, m, p, s0, ng, st->F32.p, Us, Uo, st->scal.p, stage2 ? 1 : 0, st->g32.p, st->bt32.p, st->src,
                                gyrate_close && s0 == 0 ? 1 : 0, st->src.ambi ? st->d32.p : nullptr,
                                st->src.chem && st->photo.n ? st->photo.p : nullptr, st->src.chem && st->vst.n ? st->vst.p : nullptr);
         MHD_LAUNCH_CHECK();
@@ -1213,21 +1223,21 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
                                     static_cast<float>(-(st->prm.u_inf[2] * st->prm.B_imf[0] - st->prm.u_inf[0] * st->prm.B_imf[2])),
                                     static_cast<float>(-(st->prm.u_inf[0] * st->prm.B_imf[1] - st->prm.u_inf[1] * st->prm.B_imf[0])));
     P.begin(KP_EDGE_EMF, s);
-    k_mx_edge<<<ge, 128, 0, s>>>(m, st->Ef32.p, st->up32.p, static_cast<float>(st->prm.cuct), Einf, st->E32.p);
+    launch_pdl(k_mx_edge, ge, 128, 0, s, m, st->Ef32.p, st->up32.p, static_cast<float>(st->prm.cuct), Einf, st->E32.p);
     MHD_LAUNCH_CHECK();
     if (st->src.ambi)
     {
         if (mv.nn)
-            k_mx_node_pressure<<<grid_for(mv.nn, 128), 128, 0, s>>>(mv.nn, mv.n2c_ptr, mv.n2c_cell, mv.cell_volume, W4, st->pn.p,
+            launch_pdl(k_mx_node_pressure, grid_for(mv.nn, 128), 128, 0, s, mv.nn, mv.n2c_ptr, mv.n2c_cell, mv.cell_volume, W4, st->pn.p,
                                                                     st->pok.p);
-        k_mx_ambipolar<<<grid_for(m.ne, 128), 128, 0, s>>>(m, p, W4, mv.ec_weight, mv.e_nodes, st->pn.p, st->pok.p,
+        launch_pdl(k_mx_ambipolar, grid_for(m.ne, 128), 128, 0, s, m, p, W4, mv.ec_weight, mv.e_nodes, st->pn.p, st->pok.p,
                                                             static_cast<float>(st->prm.pressure_coef), st->E32.p);
         MHD_LAUNCH_CHECK();
         st->launches += 1 + (mv.nn ? 1 : 0);
     }
     P.end(KP_EDGE_EMF, s);
     P.begin(KP_CT, s);
-    k_mx_ct<<<grid_for(m.nf, 256), 256, 0, s>>>(m.nf, st->mt.fe.p, st->E32.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
+    launch_pdl(k_mx_ct, grid_for(m.nf, 256), 256, 0, s, m.nf, st->mt.fe.p, st->E32.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
     MHD_LAUNCH_CHECK();
     P.end(KP_CT, s);
     st->launches += 3;

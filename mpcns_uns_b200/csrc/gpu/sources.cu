@@ -16,6 +16,7 @@ __global__ void __launch_bounds__(128) k_gyrate(MeshView m, SrcParams p, const d
                                                  const double *__restrict__ dtp, double scale, double dt_val, SField<double> UH,
                                                  SField<double> UN, Reprepare rp)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.no_cells || m.material[c] == 1) return;
     const double dt = dtp ? scale * *dtp : dt_val;
@@ -35,7 +36,8 @@ __global__ void __launch_bounds__(128) k_gyrate(MeshView m, SrcParams p, const d
     if (rp.on)
     {
         double u[3];
-        prepare_prims(rp.fp, rp.mass, rp.M_ref, rp.U, rp.W, c, true, u);
+        Prim5 w[2];
+        prepare_prims<2>(rp.fp, rp.mass, rp.M_ref, rp.U, rp.W, c, true, u, w);
         st3(rp.up, c, mk(u[0], u[1], u[2]));
     }
 }
@@ -62,6 +64,7 @@ __global__ void __launch_bounds__(128) k_add_sources(MeshView m, SrcParams p, in
 // electron_pressure_gradient over all cells (zero outside the owned fluid cells); W(s, c, 4) the pressures
 __global__ void __launch_bounds__(128) k_dpe(MeshView m, SField<const double> W, double *__restrict__ dpe)
 {
+    pdl_begin();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     V3 g = mk(0, 0, 0);
@@ -71,6 +74,7 @@ __global__ void __launch_bounds__(128) k_dpe(MeshView m, SField<const double> W,
 
 __global__ void __launch_bounds__(128) k_node_pressure(MeshView m, SField<const double> W, double *__restrict__ pn, int8_t *__restrict__ pok)
 {
+    pdl_begin();
     const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= m.nn) return;
     bool ok;
@@ -93,7 +97,7 @@ void launch_dpe(const MeshView &m, const double *W, double *dpe, cudaStream_t s)
 {
     if (!m.nc) return;
     const int64_t nc = m.nc;
-    k_dpe<<<grid_for(m.nc, 128), 128, 0, s>>>(m, SField<const double>{W, 5 * nc, 1, nc}, dpe);
+    launch_pdl(k_dpe, grid_for(m.nc, 128), 128, 0, s, m, SField<const double>{W, 5 * nc, 1, nc}, dpe);
     MHD_LAUNCH_CHECK();
 }
 
@@ -101,7 +105,7 @@ void launch_node_pressure(const MeshView &m, const double *W, double *pn, int8_t
 {
     if (!m.nn) return;
     const int64_t nc = m.nc;
-    k_node_pressure<<<grid_for(m.nn, 128), 128, 0, s>>>(m, SField<const double>{W, 5 * nc, 1, nc}, pn, pok);
+    launch_pdl(k_node_pressure, grid_for(m.nn, 128), 128, 0, s, m, SField<const double>{W, 5 * nc, 1, nc}, pn, pok);
     MHD_LAUNCH_CHECK();
 }
 
@@ -137,7 +141,7 @@ void launch_gyrate(const MeshView &m, const SrcParams &p, const double *B3, cons
 {
     if (!m.no_cells || !p.on || !(p.induce > 0)) return;
     const int64_t nc = m.nc;
-    k_gyrate<<<grid_for(m.no_cells, 128), 128, 0, s>>>(m, p, B3, B4, dtp, scale, 0.0, SField<double>{U, 0, 1, nc},
+    launch_pdl(k_gyrate, grid_for(m.no_cells, 128), 128, 0, s, m, p, B3, B4, dtp, scale, 0.0, SField<double>{U, 0, 1, nc},
                                                         SField<double>{U + 5 * nc, 0, 1, nc}, rp);
     MHD_LAUNCH_CHECK();
 }

@@ -190,25 +190,37 @@ __device__ __forceinline__ void gyrate_cell(const SrcParams &p, V3 b, double dt,
 }
 
 // Per-cell part of Solver::prepare (Solver.cpp:101-118): primitives of every species and the
-// charge-weighted ion velocity u+ (mhd::Scales::numinfo generalised to n species; the number
-// densities are recomputed from the primitives just written)
+// charge-weighted ion velocity u+ (mhd::Scales::numinfo generalised to n species).  NSP: the number of species, whose
+// primitives then stay in w (and go to W if store); 0: any number, the number densities recomputed from the primitives
+// just written.
+template <int NSP>
 __device__ __forceinline__ void prepare_prims(const FluidParams &p, const double *__restrict__ mass, double M_ref, SField<const double> U,
-                                              SField<double> W, int32_t c, bool fluid, double *u)
+                                              SField<double> W, int32_t c, bool fluid, double *u, Prim5 (&w)[NSP ? NSP : 1], bool store = true)
 {
     double ne = 0;
-    for (int s = 0; s < p.nsp; ++s)
+    const int nsp = NSP ? NSP : p.nsp;
+#pragma unroll
+    for (int s = 0; s < nsp; ++s)
     {
-        const Prim5 w = to_prim(U(s, c, 0), U(s, c, 1), U(s, c, 2), U(s, c, 3), U(s, c, 4), p.gamma, p.rho_floor, p.p_floor);
-        W(s, c, 0) = w.rho; W(s, c, 1) = w.u; W(s, c, 2) = w.v; W(s, c, 3) = w.w; W(s, c, 4) = w.p;
-        ne += dmax(w.rho, 0.0) / mass[s] * M_ref;
+        const Prim5 q = to_prim(U(s, c, 0), U(s, c, 1), U(s, c, 2), U(s, c, 3), U(s, c, 4), p.gamma, p.rho_floor, p.p_floor);
+        if (!NSP || store)
+        {
+            W(s, c, 0) = q.rho; W(s, c, 1) = q.u; W(s, c, 2) = q.v; W(s, c, 3) = q.w; W(s, c, 4) = q.p;
+        }
+        if (NSP) w[s] = q;
+        ne += dmax(q.rho, 0.0) / mass[s] * M_ref;
     }
     u[0] = u[1] = u[2] = 0;
     if (fluid)
-        for (int s = 0; s < p.nsp; ++s)
+#pragma unroll
+        for (int s = 0; s < nsp; ++s)
         {
-            const double ns = dmax(W(s, c, 0), 0.0) / mass[s] * M_ref;
+            const double rho = NSP ? w[s].rho : W(s, c, 0);
+            const double ns = dmax(rho, 0.0) / mass[s] * M_ref;
             const double chi = ne > 1e-300 ? ns / ne : (s == 0 ? 1.0 : 0.0);
-            for (int a = 0; a < 3; ++a) u[a] += chi * W(s, c, 1 + a);
+            u[0] += chi * (NSP ? w[s].u : W(s, c, 1));
+            u[1] += chi * (NSP ? w[s].v : W(s, c, 2));
+            u[2] += chi * (NSP ? w[s].w : W(s, c, 3));
         }
 }
 

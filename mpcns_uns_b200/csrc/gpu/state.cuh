@@ -68,6 +68,7 @@ struct MhdState
     mhd::DBuf<double> scal; // [0] dt
     mhd::DBuf<unsigned long long> dt_bits;
     mhd::DBuf<int> flag;
+    mhd::DBuf<unsigned> cfl_count; // finished blocks of the CFL pass
     // mixed precision: FP32 bulk arrays (the state U and the face fluxes Phi stay FP64)
     mhd::MixedTables mt;
     mhd::DBuf<float> W32, grad32, F32, E32;
@@ -84,6 +85,63 @@ struct MhdState
 
 namespace mhd
 {
+// Where the CFL step's minimum over the cells goes: the running minimum (bits of a positive double) and the invalid flag
+// of this step, the count of finished blocks (all three re-armed by the last block), the step size on the device, and the
+// step size and the flag in the pinned host buffer, so that the host reads them after a synchronisation without a copy.
+struct CflOut
+{
+    unsigned long long *bits;
+    int *flag;
+    unsigned *count;
+    double *dt, *host;
+    double dt_max;
+};
+inline CflOut cfl_out(const MhdState *st, double dt_max)
+{
+    return CflOut{st->dt_bits.p, st->flag.p, st->cfl_count.p, st->scal.p, st->pinned, dt_max};
+}
+#ifdef __CUDACC__
+// gdt = min(gdt, dt_max); invalid unless finite and positive (Solver.cpp:233-236)
+__device__ __forceinline__ void cfl_finish(const CflOut &o, double g, int invalid)
+{
+    g = (o.dt_max < g) ? o.dt_max : g;
+    if (!isfinite(g) || g <= 0) invalid |= 1;
+    *o.dt = g;
+    o.host[0] = g;
+    reinterpret_cast<int *>(o.host + 1)[0] = invalid;
+}
+// Block minimum of v (min is exact, so the order of the reduction does not matter), one atomic per block; the grid's last
+// block finishes the step size.  bad: a thread met a step that is zero, negative or NaN (the reference's "invalid time
+// step").  Every thread of the block calls it.
+__device__ __forceinline__ void cfl_reduce(const CflOut &o, double v, bool bad)
+{
+    constexpr double inf = 1.0 / 0.0;
+    __shared__ double sh[32];
+    __shared__ bool last;
+    for (int k = 16; k > 0; k >>= 1)
+    {
+        const double u = __shfl_xor_sync(0xffffffffu, v, k);
+        v = (u < v) ? u : v;
+    }
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    const int any = __syncthreads_or(bad);
+    if (threadIdx.x == 0)
+    {
+        for (unsigned w = 1; w < (blockDim.x >> 5); ++w) v = (sh[w] < v) ? sh[w] : v;
+        if (any) atomicOr(o.flag, 1);
+        if (v < inf) atomicMin(o.bits, static_cast<unsigned long long>(__double_as_longlong(v)));
+        __threadfence();
+        last = atomicAdd(o.count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x != 0) return;
+    __threadfence();
+    const unsigned long long b = atomicExch(o.bits, static_cast<unsigned long long>(__double_as_longlong(inf)));
+    cfl_finish(o, __longlong_as_double(static_cast<long long>(b)), atomicExch(o.flag, 0));
+    *o.count = 0;
+}
+#endif
+
 void mixed_setup(MhdState *st);
 // one FP64 stage (Us, phis) -> (Uo, phio) at the step size in st->scal[0]; stage2 averages with Uo, phio in place
 void fp64_stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2);
@@ -96,5 +154,8 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
 void mixed_gyrate_open(MhdState *st);
 void mixed_badd(MhdState *st);
 // primitives, cell fields (and with cfl the device CFL step) of (Us, phis) in mixed precision
-void mixed_prepare(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max);
+// turned: the opening gyration follows and writes the primitives and u+ of the owned fluid cells
+void mixed_prepare(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max, bool turned);
+// the CFL step of a mesh without cells: dt_max
+void cfl_empty(MhdState *st, double dt_max);
 } // namespace mhd

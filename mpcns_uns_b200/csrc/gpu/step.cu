@@ -36,99 +36,93 @@ __device__ __forceinline__ void to_cons5(const Prim5 &W, double gamma, double *U
     U[4] = W.p / (gamma - 1.0) + 0.5 * W.rho * (W.u * W.u + W.v * W.v + W.w * W.w);
 }
 
-// Solver::prepare (Solver.cpp:94-125) without the halo exchange and the cell current
-__global__ void __launch_bounds__(128) k_prepare(MeshView m, FluidParams p, const double *__restrict__ mass, double M_ref,
-                                                  SField<const double> U, SField<double> W, const double *__restrict__ phi,
-                                                  const double *__restrict__ Badd, double *__restrict__ Bind, double *__restrict__ Btot,
-                                                  double *__restrict__ up)
-{
-    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.nc) return;
-    double u[3];
-    prepare_prims(p, mass, M_ref, U, W, c, m.material[c] == 0, u);
-    const V3 b = cell_vector(m, phi, c);
-    st3(Bind, c, b);
-    st3(Btot, c, mk(b.x + Badd[3 * (int64_t)c], b.y + Badd[3 * (int64_t)c + 1], b.z + Badd[3 * (int64_t)c + 2]));
-    st3(up, c, mk(u[0], u[1], u[2]));
-}
-
+// The CFL step of one cell (mercury::cell_time_steps, MercuryUns/fluid/MercurySources.cpp:65-106, without the optional
+// gyration limit; n species: the wave speeds use the summed density, as the reference does for its two ions).  What does
+// not depend on the species is formed once per face: the face loop runs over the species inside.
+template <int NSP>
 __device__ __forceinline__ double cell_dt(const MeshView &m, const FluidParams &p, double cfl, double inver_MA2, double rho_floor_dt,
-                                          const SField<const double> &W, const double *__restrict__ Btot, int32_t c);
-
-// mercury::cell_time_steps (MercuryUns/fluid/MercurySources.cpp:65-106) without the optional gyration
-// limit, n species (the wave speeds use the summed density, as the reference does for its two ions);
-// the device-wide minimum of mercury::local_time_step (:108-116) is reduced per block first.
-__global__ void __launch_bounds__(128) k_cfl_cells(MeshView m, FluidParams p, double cfl, double inver_MA2, double rho_floor_dt,
-                                                    SField<const double> W, const double *__restrict__ Btot,
-                                                    unsigned long long *__restrict__ dt_bits, int *__restrict__ flag)
+                                          const SField<double> &W, const Prim5 (&w)[NSP ? NSP : 1], V3 b, int32_t c)
 {
-    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    double dt = CUDART_INF;
-    if (c < m.no_cells && m.material[c] == 0) dt = cell_dt(m, p, cfl, inver_MA2, rho_floor_dt, W, Btot, c);
-    if (!(dt > 0)) atomicOr(flag, 1); // zero, negative or NaN: the reference's "invalid time step"
-    // block minimum (min is exact, so the order of the reduction does not matter), one atomic per block
-    __shared__ double sh[32];
-    double v = dt > 0 ? dt : CUDART_INF;
-    for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 32)
-    {
-        v = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : CUDART_INF;
-        for (int o = 16; o > 0; o >>= 1) v = dmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (threadIdx.x == 0 && v < CUDART_INF) atomicMin(dt_bits, static_cast<unsigned long long>(__double_as_longlong(v)));
-    }
-}
-
-__device__ __forceinline__ double cell_dt(const MeshView &m, const FluidParams &p, double cfl, double inver_MA2, double rho_floor_dt,
-                                          const SField<const double> &W, const double *__restrict__ Btot, int32_t c)
-{
-    double dt = CUDART_INF;
-    const V3 b = ld3(Btot, c);
+    constexpr int MAXS = NSP ? NSP : kMaxSpecies;
+    const int nsp = NSP ? NSP : p.nsp;
     const double B2 = dot(b, b);
-    double rsum = W(0, c, 0);
-    for (int s = 1; s < p.nsp; ++s) rsum = rsum + W(s, c, 0);
-    const double rho_tot = dmax(rsum, rho_floor_dt);
-    const int32_t k0 = m.c2f_ptr[c], k1 = m.c2f_ptr[c + 1];
-    for (int s = 0; s < p.nsp; ++s)
+    double rsum = NSP ? w[0].rho : W(0, c, 0);
+#pragma unroll
+    for (int s = 1; s < nsp; ++s) rsum = rsum + (NSP ? w[s].rho : W(s, c, 0));
+    const double rho_tot = dmax(rsum, rho_floor_dt), vA2 = inver_MA2 * B2 / rho_tot;
+    double cs2[MAXS], denom[MAXS];
+#pragma unroll
+    for (int s = 0; s < nsp; ++s)
     {
-        const double cs2 = p.gamma * W(s, c, 4) / dmax(W(s, c, 0), 1e-30);
-        double denom = 0;
-        for (int32_t k = k0; k < k1; ++k)
-        {
-            const int32_t f = m.c2f_idx[k];
-            const double A = m.face_area_mag[f];
-            const V3 n = (1.0 / A) * ld3(m.face_area, f);
-            const double vA2 = inver_MA2 * B2 / rho_tot;
-            const double vAn2 = inver_MA2 * dot(b, n) * dot(b, n) / rho_tot;
-            const double term = cs2 + vA2;
-            const double cf = sqrt(0.5 * (term + sqrt(dmax(0.0, term * term - 4 * cs2 * vAn2))));
-            denom += (fabs(W(s, c, 1) * n.x + W(s, c, 2) * n.y + W(s, c, 3) * n.z) + cf) * A;
-        }
-        if (denom > 0) dt = dmin(dt, cfl * m.cell_volume[c] / denom);
+        cs2[s] = p.gamma * (NSP ? w[s].p : W(s, c, 4)) / dmax(NSP ? w[s].rho : W(s, c, 0), 1e-30);
+        denom[s] = 0;
     }
+    const int32_t k0 = m.c2f_ptr[c], k1 = m.c2f_ptr[c + 1];
+    for (int32_t k = k0; k < k1; ++k)
+    {
+        const D4 n4 = ld_d4(m.fna + 4 * (int64_t)m.c2f_idx[k]);
+        const V3 n = mk(n4.x, n4.y, n4.z);
+        const double A = n4.w, bn = dot(b, n), vAn2 = inver_MA2 * bn * bn / rho_tot;
+#pragma unroll
+        for (int s = 0; s < nsp; ++s)
+        {
+            const double u = NSP ? w[s].u : W(s, c, 1), v = NSP ? w[s].v : W(s, c, 2), z = NSP ? w[s].w : W(s, c, 3);
+            const double term = cs2[s] + vA2;
+            const double cf = sqrt(0.5 * (term + sqrt(dmax(0.0, term * term - 4 * cs2[s] * vAn2))));
+            denom[s] += (fabs(u * n.x + v * n.y + z * n.z) + cf) * A;
+        }
+    }
+    double dt = CUDART_INF;
+#pragma unroll
+    for (int s = 0; s < nsp; ++s)
+        if (denom[s] > 0) dt = dmin(dt, cfl * m.cell_volume[c] / denom[s]);
     return dt;
 }
 
-__global__ void k_cfl_init(unsigned long long *dt_bits, int *flag)
+struct CflArgs
 {
-    *dt_bits = static_cast<unsigned long long>(__double_as_longlong(CUDART_INF));
-    *flag = 0;
+    double cfl, inver_MA2, rho_floor_dt;
+    int turned; // the opening gyration follows: it writes W and up of the owned fluid cells itself
+    CflOut out;
+};
+
+// Solver::prepare (Solver.cpp:94-125) without the halo exchange and the cell current.  CFL: with the step size of
+// mercury::local_time_step (MercurySources.cpp:108-116) from the values at hand, its minimum finished by the last block
+// (1.77M tetrahedra, two species: 188 us, 138 + 179 as two passes, and three launches less).
+template <int NSP, bool CFL>
+__global__ void __launch_bounds__(128) k_prepare(MeshView m, FluidParams p, const double *__restrict__ mass, double M_ref,
+                                                  SField<const double> U, SField<double> W, const double *__restrict__ phi,
+                                                  const double *__restrict__ Badd, double *__restrict__ Bind, double *__restrict__ Btot,
+                                                  double *__restrict__ up, CflArgs cfl)
+{
+    pdl_begin();
+    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    double dt = CUDART_INF;
+    if (c < m.nc)
+    {
+        double u[3];
+        Prim5 w[NSP ? NSP : 1];
+        const bool fluid = m.material[c] == 0;
+        const bool store = !CFL || !cfl.turned || c >= m.no_cells || m.material[c] == 1;
+        prepare_prims<NSP>(p, mass, M_ref, U, W, c, fluid, u, w, store);
+        const V3 b = cell_vector(m, phi, c);
+        const V3 bt = mk(b.x + Badd[3 * (int64_t)c], b.y + Badd[3 * (int64_t)c + 1], b.z + Badd[3 * (int64_t)c + 2]);
+        st3(Bind, c, b);
+        st3(Btot, c, bt);
+        if (store) st3(up, c, mk(u[0], u[1], u[2]));
+        if (CFL && c < m.no_cells && fluid) dt = cell_dt<NSP>(m, p, cfl.cfl, cfl.inver_MA2, cfl.rho_floor_dt, W, w, bt, c);
+    }
+    if constexpr (CFL) cfl_reduce(cfl.out, dt > 0 ? dt : CUDART_INF, !(dt > 0));
 }
 
-// gdt = min(gdt, dt_max); invalid unless finite and positive (Solver.cpp:233-236)
-__global__ void k_cfl_final(const unsigned long long *dt_bits, double dt_max, double *dt, int *flag)
-{
-    double g = __longlong_as_double(static_cast<long long>(*dt_bits));
-    g = dmin(g, dt_max);
-    if (!isfinite(g) || g <= 0) atomicOr(flag, 1);
-    *dt = g;
-}
+// the step size of a mesh without cells
+__global__ void k_cfl_empty(CflOut o) { cfl_finish(o, CUDART_INF, 0); }
 
-__global__ void k_set_dt(double *dt, double v, int *flag)
+__global__ void k_set_dt(double *dt, double v, double *host)
 {
     *dt = v;
-    *flag = 0;
+    host[0] = v;
+    reinterpret_cast<int *>(host + 1)[0] = 0;
 }
 
 // Inputs of the two-ion J x B source added to the gathered rhs (mercury::Solver::rhs, Solver.cpp:146-149)
@@ -144,16 +138,18 @@ struct SrcView
 // reference's scatter order, plus the J x B source when it is on, U = U_base + dt rhs on the owned
 // fluid cells, Solver::enforce_floors (:171-191); stage 2 averages with U0 in place (Solver.cpp:505-506).
 // NF = 4: tetrahedral mesh, the four faces of the cell unrolled (all flux gathers in flight together);
-// NF = 0: any polyhedra.  One thread per (cell, species of the group = blockIdx.y).
+// NF = 6 likewise; NF = 0: any polyhedra.  One thread per (cell, species of the group); the species of a cell in
+// neighbouring blocks, which share its rows and sources.
 // fl (optional): which floor each owned fluid cell and species met, [s*nc + c]: 0 none, 1 density, 2 pressure.
 template <int NF>
 __global__ void __launch_bounds__(128) k_update(MeshView m, FluidParams p, int s0, int ng, const double *__restrict__ F,
                                                  SField<const double> Ub, SField<double> Uo, const double *__restrict__ dtp, int stage2,
                                                  SrcView sv, int8_t *__restrict__ fl)
 {
-    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int g = blockIdx.y;
-    if (c >= m.nc || g >= ng) return;
+    pdl_begin();
+    const int g = blockIdx.x % ng;
+    const int32_t c = (blockIdx.x / ng) * blockDim.x + threadIdx.x;
+    if (c >= m.nc) return;
     const int64_t nf = m.nf;
     const double dt = *dtp;
     const bool live = c < m.no_cells && m.material[c] == 0;
@@ -166,19 +162,33 @@ __global__ void __launch_bounds__(128) k_update(MeshView m, FluidParams p, int s
         if (live)
         {
             double r[5] = {0, 0, 0, 0, 0};
-            if constexpr (NF == 4)
+            if constexpr (NF > 0)
             {
-                const int4 fi = *reinterpret_cast<const int4 *>(m.cfa_idx + k0);
-                const char4 sg = *reinterpret_cast<const char4 *>(m.cfa_sgn + k0);
-                const int32_t ff[4] = {fi.x, fi.y, fi.z, fi.w};
-                const bool out[4] = {sg.x > 0, sg.y > 0, sg.z > 0, sg.w > 0};
-                double Fv[4][5];
+                int32_t ff[NF];
+                bool out[NF];
+                if constexpr (NF == 4)
+                {
+                    const int4 fi = *reinterpret_cast<const int4 *>(m.cfa_idx + k0);
+                    const char4 sg = *reinterpret_cast<const char4 *>(m.cfa_sgn + k0);
+                    ff[0] = fi.x; ff[1] = fi.y; ff[2] = fi.z; ff[3] = fi.w;
+                    out[0] = sg.x > 0; out[1] = sg.y > 0; out[2] = sg.z > 0; out[3] = sg.w > 0;
+                }
+                else
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < NF; j += 2)
+                    {
+                        const int2 fi = *reinterpret_cast<const int2 *>(m.cfa_idx + k0 + j);
+                        const char2 sg = *reinterpret_cast<const char2 *>(m.cfa_sgn + k0 + j);
+                        ff[j] = fi.x; ff[j + 1] = fi.y;
+                        out[j] = sg.x > 0; out[j + 1] = sg.y > 0;
+                    }
+                double Fv[NF][5];
+#pragma unroll
+                for (int j = 0; j < NF; ++j)
 #pragma unroll
                     for (int q = 0; q < 5; ++q) Fv[j][q] = F[(g * 5 + q) * nf + ff[j]];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < NF; ++j)
 #pragma unroll
                     for (int q = 0; q < 5; ++q)
                     {
@@ -232,6 +242,7 @@ __global__ void __launch_bounds__(128) k_update(MeshView m, FluidParams p, int s
 __global__ void __launch_bounds__(256) k_ct(MeshView m, const double *__restrict__ E, const double *__restrict__ phis,
                                              double *__restrict__ phio, const double *__restrict__ dtp, int stage2)
 {
+    pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nf) return;
     bool active = false;
@@ -293,21 +304,32 @@ namespace
 SField<double> soa_state(double *p, int64_t nc) { return {p, 5 * nc, 1, nc}; }
 SField<const double> soa_cstate(const double *p, int64_t nc) { return {p, 5 * nc, 1, nc}; }
 
+// k_prepare over every cell, with the CFL step when cfl
+void launch_prepare(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max, bool turned = false)
+{
+    const MeshView &m = st->mesh->v;
+    const int64_t nc = m.nc;
+    const CflArgs ca{st->prm.cfl, st->prm.inver_MA2, st->prm.rho_floor_dt, turned ? 1 : 0, cfl_out(st, dt_max)};
+    auto k = st->nsp == 1 ? (cfl ? k_prepare<1, true> : k_prepare<1, false>)
+             : st->nsp == 2 ? (cfl ? k_prepare<2, true> : k_prepare<2, false>)
+                            : (cfl ? k_prepare<0, true> : k_prepare<0, false>);
+    launch_pdl(k, grid_for(m.nc, 128), 128, 0, st->mesh->stream, m, st->fp, st->mass.p, st->prm.M_ref, soa_cstate(Us, nc),
+               soa_state(st->W.p, nc), phis, st->badd.p, st->bind.p, st->btot.p, st->up.p, ca);
+}
+
 // Solver::prepare of (Us, phis) (with the cell current when the J x B force is on) and, with cfl,
 // the device CFL step (mercury::local_time_step) into scal[0]
-void prepare_cfl(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max)
+void prepare_cfl(MhdState *st, const double *Us, const double *phis, bool cfl, double dt_max, bool turned = false)
 {
     MhdMesh *mesh = st->mesh;
     const MeshView &m = mesh->v;
     cudaStream_t s = mesh->stream;
-    const int64_t nc = m.nc;
     Profiler &P = st->prof;
     if (m.nc)
     {
         P.begin(KP_PREPARE, s);
-        k_prepare<<<grid_for(m.nc, 128), 128, 0, s>>>(m, st->fp, st->mass.p, st->prm.M_ref, soa_cstate(Us, nc), soa_state(st->W.p, nc),
-                                                      phis, st->badd.p, st->bind.p, st->btot.p, st->up.p);
-        MHD_LAUNCH_CHECK();
+        // grad p_e and the nodal p_e below need the primitives before the gyration
+        launch_prepare(st, Us, phis, cfl, dt_max, turned && !st->src.ambi);
         ++st->launches;
         if (st->src.on) // J of the induced field (Solver.cpp:123)
         {
@@ -322,18 +344,7 @@ void prepare_cfl(MhdState *st, const double *Us, const double *phis, bool cfl, d
         }
         P.end(KP_PREPARE, s);
     }
-    if (cfl)
-    {
-        P.begin(KP_CFL, s);
-        k_cfl_init<<<1, 1, 0, s>>>(st->dt_bits.p, st->flag.p);
-        if (m.no_cells)
-            k_cfl_cells<<<grid_for(m.no_cells, 128), 128, 0, s>>>(m, st->fp, st->prm.cfl, st->prm.inver_MA2, st->prm.rho_floor_dt,
-                                                                   soa_cstate(st->W.p, nc), st->btot.p, st->dt_bits.p, st->flag.p);
-        k_cfl_final<<<1, 1, 0, s>>>(st->dt_bits.p, dt_max, st->scal.p, st->flag.p);
-        MHD_LAUNCH_CHECK();
-        P.end(KP_CFL, s);
-        st->launches += m.no_cells ? 3 : 2;
-    }
+    else if (cfl) cfl_empty(st, dt_max);
 }
 
 void stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2, bool cfl, double dt_max,
@@ -383,13 +394,9 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
         if (m.nc)
         {
             P.begin(KP_UPDATE, s);
-            const dim3 grid(grid_for(m.nc, 128), ng);
-            if (m.faces_per_cell == 4)
-                k_update<4><<<grid, 128, 0, s>>>(m, st->fp, s0, ng, st->F.p, soa_cstate(Us, nc), soa_state(Uo, nc), st->scal.p,
-                                                 stage2 ? 1 : 0, sv, st->floor_flags);
-            else
-                k_update<0><<<grid, 128, 0, s>>>(m, st->fp, s0, ng, st->F.p, soa_cstate(Us, nc), soa_state(Uo, nc), st->scal.p,
-                                                 stage2 ? 1 : 0, sv, st->floor_flags);
+            launch_pdl(m.faces_per_cell == 4 ? k_update<4> : m.faces_per_cell == 6 ? k_update<6> : k_update<0>,
+                       grid_for(m.nc, 128) * ng, 128, 0, s, m, st->fp, s0, ng, st->F.p, soa_cstate(Us, nc), soa_state(Uo, nc), st->scal.p,
+                       stage2 ? 1 : 0, sv, st->floor_flags);
             MHD_LAUNCH_CHECK();
             P.end(KP_UPDATE, s);
         }
@@ -415,7 +422,7 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
     if (ct && m.nf)
     {
         P.begin(KP_CT, s);
-        k_ct<<<grid_for(m.nf, 256), 256, 0, s>>>(m, st->E.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
+        launch_pdl(k_ct, grid_for(m.nf, 256), 256, 0, s, m, st->E.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
         MHD_LAUNCH_CHECK();
         P.end(KP_CT, s);
         ++st->launches;
@@ -423,6 +430,13 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
 }
 
 } // namespace
+
+void cfl_empty(MhdState *st, double dt_max)
+{
+    k_cfl_empty<<<1, 1, 0, st->mesh->stream>>>(cfl_out(st, dt_max));
+    MHD_LAUNCH_CHECK();
+    ++st->launches;
+}
 
 // One FP64 stage at the step size already in st->scal[0] (no CFL), for the differentiated run
 void fp64_stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2)
@@ -449,9 +463,7 @@ namespace
 void read_dt(MhdState *st, double *dt_host)
 {
     cudaStream_t s = st->mesh->stream;
-    MHD_CUDA(cudaMemcpyAsync(st->pinned, st->scal.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-    MHD_CUDA(cudaMemcpyAsync(st->pinned + 1, st->flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MHD_CUDA(cudaStreamSynchronize(s));
+    MHD_CUDA(cudaStreamSynchronize(s)); // the step's kernels wrote the step size and the flag to the pinned buffer
     int flag;
     std::memcpy(&flag, st->pinned + 1, sizeof(int));
     if (flag) throw ApiError(MHD_ESTATE, "invalid time step");
@@ -551,6 +563,7 @@ int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *p, MhdState **out)
         st->scal.alloc(4);
         st->dt_bits.alloc(1);
         st->flag.alloc(1);
+        st->cfl_count.alloc(1);
         st->mass.upload(p->mass, st->nsp);
         st->src = src_params(*p);
         if (st->src.on) st->J.alloc(3 * nc);
@@ -592,6 +605,9 @@ int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *p, MhdState **out)
         }
         if (nc) MHD_CUDA(cudaMemsetAsync(st->badd.p, 0, 3 * nc * sizeof(double), s));
         MHD_CUDA(cudaMemsetAsync(st->flag.p, 0, sizeof(int), s));
+        MHD_CUDA(cudaMemsetAsync(st->cfl_count.p, 0, sizeof(unsigned), s));
+        const double inf = HUGE_VAL;
+        MHD_CUDA(cudaMemcpyAsync(st->dt_bits.p, &inf, sizeof(inf), cudaMemcpyHostToDevice, s));
         MHD_CUDA(cudaStreamSynchronize(s));
         *out = st;
     });
@@ -710,17 +726,8 @@ int mhd_gpu_cfl_dt(MhdState *st, double dt_max, double *host_dt)
         MHD_REQUIRE(st && host_dt, "null argument");
         MhdMesh *mesh = st->mesh;
         const MeshView &m = mesh->v;
-        cudaStream_t s = mesh->stream;
-        const int64_t nc = m.nc;
-        if (nc)
-            k_prepare<<<grid_for(m.nc, 128), 128, 0, s>>>(m, st->fp, st->mass.p, st->prm.M_ref, soa_cstate(st->U0.p, nc),
-                                                          soa_state(st->W.p, nc), st->phi0.p, st->badd.p, st->bind.p, st->btot.p,
-                                                          st->up.p);
-        k_cfl_init<<<1, 1, 0, s>>>(st->dt_bits.p, st->flag.p);
-        if (m.no_cells)
-            k_cfl_cells<<<grid_for(m.no_cells, 128), 128, 0, s>>>(m, st->fp, st->prm.cfl, st->prm.inver_MA2, st->prm.rho_floor_dt,
-                                                                   soa_cstate(st->W.p, nc), st->btot.p, st->dt_bits.p, st->flag.p);
-        k_cfl_final<<<1, 1, 0, s>>>(st->dt_bits.p, dt_max, st->scal.p, st->flag.p);
+        if (m.nc) launch_prepare(st, st->U0.p, st->phi0.p, true, dt_max);
+        else cfl_empty(st, dt_max);
         MHD_LAUNCH_CHECK();
         read_dt(st, host_dt);
     });
@@ -735,7 +742,7 @@ int mhd_gpu_step_rk2(MhdState *st, double dt_fixed, double dt_max, double *dt_us
         const bool cfl = !(dt_fixed > 0);
         if (!cfl)
         {
-            k_set_dt<<<1, 1, 0, s>>>(st->scal.p, dt_fixed, st->flag.p);
+            k_set_dt<<<1, 1, 0, s>>>(st->scal.p, dt_fixed, st->pinned);
             MHD_LAUNCH_CHECK();
             ++st->launches;
         }
@@ -748,7 +755,7 @@ int mhd_gpu_step_rk2(MhdState *st, double dt_fixed, double dt_max, double *dt_us
         {
             if (split)
             {
-                mixed_prepare(st, st->U0.p, st->phi0.p, cfl, dt_max);
+                mixed_prepare(st, st->U0.p, st->phi0.p, cfl, dt_max, true);
                 st->prof.begin(KP_GYRATE, s);
                 mixed_gyrate_open(st);
                 st->prof.end(KP_GYRATE, s);
@@ -760,7 +767,7 @@ int mhd_gpu_step_rk2(MhdState *st, double dt_fixed, double dt_max, double *dt_us
         {
             if (split)
             {
-                prepare_cfl(st, st->U0.p, st->phi0.p, cfl, dt_max);
+                prepare_cfl(st, st->U0.p, st->phi0.p, cfl, dt_max, true);
                 // the gyration renews the primitives and u+ of the cells it turns: stage 1 starts prepared
                 Reprepare rp;
                 rp.on = 1;
@@ -805,7 +812,7 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
         const bool cfl = !(dt_fixed > 0);
         if (!cfl)
         {
-            k_set_dt<<<1, 1, 0, s>>>(st->scal.p, dt_fixed, st->flag.p);
+            k_set_dt<<<1, 1, 0, s>>>(st->scal.p, dt_fixed, st->pinned);
             MHD_LAUNCH_CHECK();
             ++st->launches;
         }
@@ -814,7 +821,7 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
         const bool split = st->src.on && st->src.induce > 0;
         if (split)
         {
-            prepare_cfl(st, st->U0.p, st->phi0.p, cfl, dt_max);
+            prepare_cfl(st, st->U0.p, st->phi0.p, cfl, dt_max, true);
             Reprepare rp;
             rp.on = 1;
             rp.fp = st->fp;
@@ -862,7 +869,7 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
         if (m.nf)
         {
             st->prof.begin(KP_CT, s);
-            k_ct<<<grid_for(m.nf, 256), 256, 0, s>>>(m, st->E_impl.p, st->phi0.p, st->phi0.p, st->scal.p, 0);
+            launch_pdl(k_ct, grid_for(m.nf, 256), 256, 0, s, m, st->E_impl.p, st->phi0.p, st->phi0.p, st->scal.p, 0);
             MHD_LAUNCH_CHECK();
             st->prof.end(KP_CT, s);
             ++st->launches;
