@@ -144,6 +144,10 @@ int mhd_gpu_mesh_destroy(MhdMesh *mesh);
 /* The CUDA stream (cudaStream_t) the handle's work is ordered on; may be replaced by the caller's. */
 void *mhd_gpu_mesh_stream(MhdMesh *mesh);
 int mhd_gpu_mesh_set_stream(MhdMesh *mesh, void *stream);
+/* Order the handle's stream after the work enqueued on `stream` so far, and `stream` after the handle's: what a caller
+ * whose arrays are produced and consumed on a stream of its own puts around the calls.  Neither waits on the host. */
+int mhd_gpu_mesh_wait_stream(MhdMesh *mesh, void *stream);
+int mhd_gpu_stream_wait_mesh(MhdMesh *mesh, void *stream);
 int mhd_gpu_synchronize(MhdMesh *mesh);
 
 /* mhd::to_prim over n cells (Common/physics/Euler.h:13-21): U, W 5 per cell. */

@@ -471,6 +471,53 @@ int mhd_gpu_mesh_set_stream(MhdMesh *mesh, void *stream)
     });
 }
 
+namespace
+{
+// The calling thread's event of the current device for ordering two streams: recorded and waited on at once, so one
+// event serves every call of the thread (a wait keeps the state that the event had when it was enqueued).
+struct ThreadEvents
+{
+    std::vector<cudaEvent_t> ev;
+    ~ThreadEvents()
+    {
+        for (cudaEvent_t e : ev)
+            if (e) cudaEventDestroy(e);
+    }
+    cudaEvent_t get()
+    {
+        int dev = 0;
+        MHD_CUDA(cudaGetDevice(&dev));
+        if (ev.size() <= (size_t)dev) ev.resize(dev + 1, nullptr);
+        if (!ev[dev]) MHD_CUDA(cudaEventCreateWithFlags(&ev[dev], cudaEventDisableTiming));
+        return ev[dev];
+    }
+};
+void stream_after(cudaStream_t later, cudaStream_t earlier)
+{
+    static thread_local ThreadEvents events;
+    if (later == earlier) return;
+    const cudaEvent_t e = events.get();
+    MHD_CUDA(cudaEventRecord(e, earlier));
+    MHD_CUDA(cudaStreamWaitEvent(later, e, 0));
+}
+} // namespace
+
+int mhd_gpu_mesh_wait_stream(MhdMesh *mesh, void *stream)
+{
+    return guarded([&] {
+        MHD_REQUIRE(mesh, "null mesh");
+        stream_after(mesh->stream, static_cast<cudaStream_t>(stream));
+    });
+}
+
+int mhd_gpu_stream_wait_mesh(MhdMesh *mesh, void *stream)
+{
+    return guarded([&] {
+        MHD_REQUIRE(mesh, "null mesh");
+        stream_after(static_cast<cudaStream_t>(stream), mesh->stream);
+    });
+}
+
 int mhd_gpu_synchronize(MhdMesh *mesh)
 {
     return guarded([&] {

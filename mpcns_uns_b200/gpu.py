@@ -79,6 +79,8 @@ _SIGS = {
     "mhd_gpu_mesh_stream": ([vp], vp),
     "mhd_gpu_mesh_set_stream": ([vp, vp], ctypes.c_int),
     "mhd_gpu_synchronize": ([vp], ctypes.c_int),
+    "mhd_gpu_mesh_wait_stream": ([vp, vp], ctypes.c_int),
+    "mhd_gpu_stream_wait_mesh": ([vp, vp], ctypes.c_int),
     "mhd_gpu_to_prim": ([vp, vp, i32, dbl, dbl, dbl, vp], ctypes.c_int),
     "mhd_gpu_limited_gradients": ([vp, vp, i32, ctypes.POINTER(Prim), i32, dbl, vp], ctypes.c_int),
     "mhd_gpu_flux_rhs": ([vp, dbl, i32, ctypes.POINTER(Prim), vp, vp, vp], ctypes.c_int),
@@ -180,11 +182,17 @@ def check(rc):
         raise MhdError(rc, lib().mhd_gpu_last_error().decode())
 
 
+_torch_cuda = None   # torch, once it has been seen with a CUDA device
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("mpcns_uns_b200.gpu needs a CUDA device (no CPU fallback)")
-    return torch
+    global _torch_cuda
+    if _torch_cuda is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("mpcns_uns_b200.gpu needs a CUDA device (no CPU fallback)")
+        _torch_cuda = torch
+    return _torch_cuda
 
 
 def dev(a, dtype=None):
@@ -262,10 +270,10 @@ class DeviceMesh:
 
     def _enter(self):
         # the handle's stream must see every tensor that torch's current stream produced
-        self._stream.wait_stream(_torch().cuda.current_stream())
+        check(lib().mhd_gpu_mesh_wait_stream(self._h, _torch().cuda.current_stream().cuda_stream))
 
     def _leave(self):
-        _torch().cuda.current_stream().wait_stream(self._stream)
+        check(lib().mhd_gpu_stream_wait_mesh(self._h, _torch().cuda.current_stream().cuda_stream))
 
     # ------------------------------------------------------------- reference functions
     def to_prim(self, U, gamma, rho_floor=1e-10, p_floor=1e-12):
