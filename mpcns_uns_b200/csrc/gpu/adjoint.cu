@@ -578,20 +578,22 @@ __global__ void k_a_J(MeshView m, const double *__restrict__ phi, const double *
 // y_c = I_c^T lB_c (the transpose of the cell fit B_c = I_c sum_k n_k Phi_k); lB is cleared for the next stage
 __device__ __forceinline__ V3 recon_T(const MeshView &m, int32_t c, V3 lb)
 {
-    double I[3][3];
-    if (!cell_vector_inverse(m, c, I)) return mk(0, 0, 0);
-    return mk(I[0][0] * lb.x + I[1][0] * lb.y + I[2][0] * lb.z, I[0][1] * lb.x + I[1][1] * lb.y + I[2][1] * lb.z,
-              I[0][2] * lb.x + I[1][2] * lb.y + I[2][2] * lb.z);
+    const int64_t n = m.nc;
+    const double *I = m.cinv + c;
+    return mk(I[0] * lb.x + I[3 * n] * lb.y + I[6 * n] * lb.z, I[n] * lb.x + I[4 * n] * lb.y + I[7 * n] * lb.z,
+              I[2 * n] * lb.x + I[5 * n] * lb.y + I[8 * n] * lb.z);
 }
 
 // lphi_f += n_f . (y_L + y_R), n_f = A_f / |A_f| (faces with |A_f| > 0)
 __device__ __forceinline__ double recon_T_face(const MeshView &m, const double *__restrict__ y, int32_t f)
 {
-    const double A = m.face_area_mag[f];
-    if (A <= 0) return 0.0;
-    const V3 n = (1.0 / A) * ld3(m.face_area, f);
+    const D4 n4 = ld_d4(m.fna + 4 * (int64_t)f);
+    if (n4.w <= 0) return 0.0;
+    const V3 n = mk(n4.x, n4.y, n4.z);
+    const int32_t L = m.face_L[f], R = m.face_R[f];
     double acc = 0.0;
-    for (int32_t k = m.f2c_ptr[f]; k < m.f2c_ptr[f + 1]; ++k) acc += mhd::dot(n, ld3(y, m.f2c_idx[k]));
+    if (L >= 0) acc += mhd::dot(n, ld3(y, L));
+    if (R >= 0) acc += mhd::dot(n, ld3(y, R));
     return acc;
 }
 
@@ -1008,51 +1010,44 @@ __device__ __forceinline__ void ghost_T(int kind, bool absorb, V3 n, const doubl
 }
 
 // K4: face adjoint of the flux and its gather, per (face, species): lF = sum over the face's cells of -/+ lrV,
-// the reverse Rusanov flux, the ghost state; writes the adjoint of each cell's face state into its slot
-// lface[((s*2 + side)*5 + q)*nf + f] (side 0: the cell with c2f sign +1).  Species 0 also adds the cell-fit
-// transpose n_f . (y_L + y_R) to lphi.
-__global__ void __launch_bounds__(128) k_a_flux(MeshView m, FluidParams p, const double *__restrict__ W, const double *__restrict__ G,
-                                                 const double *__restrict__ lrV, double *__restrict__ lface, double *__restrict__ lfs,
-                                                 const double *__restrict__ y, double *__restrict__ lphi)
+// the reverse Rusanov flux at the face values FV that the forward stage left, the ghost state; writes the adjoint of each
+// cell's face state into its slot lface[((s*2 + side)*5 + q)*nf + f] (side 0: the cell with c2f sign +1).  Species 0
+// also adds the cell-fit transpose n_f . (y_L + y_R) to lphi.
+// 295k tetrahedra, two species: 76 us, 94 from the gradients.
+__global__ void __launch_bounds__(128) k_a_flux(MeshView m, FluidParams p, const double *__restrict__ FV, const double *__restrict__ lrV,
+                                                 double *__restrict__ lface, double *__restrict__ lfs, const double *__restrict__ y,
+                                                 double *__restrict__ lphi)
 {
-    const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    const int s = blockIdx.y;
-    if (f >= m.nf || s >= p.nsp) return;
-    const int64_t nf = m.nf, n = m.nc;
+    const int s = blockIdx.x % p.nsp;
+    const int32_t f = (blockIdx.x / p.nsp) * blockDim.x + threadIdx.x;
+    if (f >= m.nf) return;
+    const int64_t nf = m.nf, n = m.nc, nnz = 4 * n;
     if (s == 0) lphi[f] += recon_T_face(m, y, f);
     double *o0 = lface + (int64_t)(s * 2) * 5 * nf + f, *o1 = lface + (int64_t)(s * 2 + 1) * 5 * nf + f;
-    const int kind = m.face_kind[f];
-    const int32_t p0 = m.f2c_ptr[f], cnt = m.f2c_ptr[f + 1] - p0;
-    bool any_owned = false;
+    const int4 r = m.frec[f];
+    const int type = r.z & 15;
+    const int32_t cL = m.face_L[f], cR = m.face_R[f];
     double lF[5] = {0, 0, 0, 0, 0};
-    for (int k = 0; k < cnt; ++k)
-    {
-        const int32_t cc = m.f2c_idx[p0 + k];
-        any_owned |= cc < m.no_cells && m.material[cc] == 0;
-        const double sg = m.f2c_sgn[p0 + k] > 0 ? -1.0 : 1.0;
-        for (int q = 0; q < 5; ++q) lF[q] += sg * lrV[ui(s, q, cc, n)];
-    }
+    if (cL >= 0)
+        for (int q = 0; q < 5; ++q) lF[q] += -lrV[ui(s, q, cL, n)];
+    if (cR >= 0)
+        for (int q = 0; q < 5; ++q) lF[q] += lrV[ui(s, q, cR, n)];
     const bool zero = lF[0] == 0.0 && lF[1] == 0.0 && lF[2] == 0.0 && lF[3] == 0.0 && lF[4] == 0.0;
-    if (kind == 4 || !any_owned || zero)
+    if (type == FF_NONE || zero)
     {
         for (int q = 0; q < 5; ++q) o0[q * nf] = o1[q * nf] = 0.0;
         return;
     }
-    const double A = m.face_area_mag[f];
-    for (int q = 0; q < 5; ++q) lF[q] *= A;
-    const V3 nv = (1.0 / A) * ld3(m.face_area, f);
-    const V3 xf = ld3(m.face_center, f);
-    auto state_of = [&](int32_t cc) {
-        const Prim5 w{W[ui(s, 0, cc, n)], W[ui(s, 1, cc, n)], W[ui(s, 2, cc, n)], W[ui(s, 3, cc, n)], W[ui(s, 4, cc, n)]};
-        double g[15];
-        for (int q = 0; q < 15; ++q) g[q] = G[gi(s, q, cc, n)];
-        return face_state(w, g, xf - ld3(m.cell_center, cc));
-    };
+    const D4 n4 = ld_d4(m.fna + 4 * (int64_t)f);
+    for (int q = 0; q < 5; ++q) lF[q] *= n4.w;
+    const V3 nv = mk(n4.x, n4.y, n4.z);
+    const double *fv = FV + s * 5 * nnz;
+    auto state = [&](int32_t k) { return Prim5{fv[k], fv[nnz + k], fv[2 * nnz + k], fv[3 * nnz + k], fv[4 * nnz + k]}; };
     double lL[5], lR[5];
-    if (cnt == 2 && kind == 0)
+    const Prim5 in = state(r.x);
+    if (type == FF_INTERIOR)
     {
-        const Prim5 L = state_of(m.face_L[f]), R = state_of(m.face_R[f]);
-        rusanov_T(L, R, nv, p.gamma, lF, lL, lR);
+        rusanov_T(in, state(r.y), nv, p.gamma, lF, lL, lR);
         for (int q = 0; q < 5; ++q)
         {
             o0[q * nf] = lL[q];
@@ -1060,27 +1055,15 @@ __global__ void __launch_bounds__(128) k_a_flux(MeshView m, FluidParams p, const
         }
         return;
     }
-    int32_t c = m.f2c_idx[p0];
-    int sgn = m.f2c_sgn[p0];
-    if (cnt == 2 && m.material[c] != 0)
-    {
-        c = m.f2c_idx[p0 + 1];
-        sgn = m.f2c_sgn[p0 + 1];
-    }
-    const Prim5 in = state_of(c);
-    const V3 nn = double(sgn) * nv;
+    const int kind = r.z >> 4;
+    const bool left = type == FF_INSIDE_L;
+    const V3 nn = (left ? 1.0 : -1.0) * nv;
     const Prim5 gh = ghost_state(kind, p.absorb[s] != 0, in, nn, p.fs[s]);
     double lin[5], lg[5];
-    if (sgn > 0)
-    {
-        rusanov_T(in, gh, nv, p.gamma, lF, lin, lg);
-    }
-    else
-    {
-        rusanov_T(gh, in, nv, p.gamma, lF, lg, lin);
-    }
+    if (left) rusanov_T(in, gh, nv, p.gamma, lF, lin, lg);
+    else rusanov_T(gh, in, nv, p.gamma, lF, lg, lin);
     ghost_T(kind, p.absorb[s] != 0, nn, lg, lin, lfs + 5 * s);
-    double *mine = sgn > 0 ? o0 : o1, *other = sgn > 0 ? o1 : o0;
+    double *mine = left ? o0 : o1, *other = left ? o1 : o0;
     for (int q = 0; q < 5; ++q)
     {
         mine[q * nf] = lin[q];
@@ -1088,174 +1071,209 @@ __global__ void __launch_bounds__(128) k_a_flux(MeshView m, FluidParams p, const
     }
 }
 
-// K5: per (cell, species): the face-state transpose (lW, lG from the cell's four face slots), then the
-// reverse of k_limited_gradients_tet.  lW holds the u+ part on entry and the cell's own total on exit;
-// slot[((s*4 + j)*5 + q)*nc + c] receives the adjoint of neighbour j's primitive q as this cell's stencil saw it.
-// Every loop over the four slots and five variables is unrolled and the winning slots of the min / max
-// terms are selected by predicates, so the per-thread arrays stay in registers.
-__global__ void __launch_bounds__(128, 3) k_a_grad(MeshView m, FluidParams p, const double *__restrict__ W, const double *__restrict__ G,
-                                                 const double *__restrict__ lface, double *__restrict__ lW, double *__restrict__ slot,
-                                                 double *__restrict__ lfs)
+// one component of ghost_state (q = 0..4), wc the inside state's
+__device__ __forceinline__ double ghost_q(int kind, bool absorb, int q, const double *w, V3 n, const Prim5 &fs)
 {
-    const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int s = blockIdx.y;
-    if (c >= m.nc || s >= p.nsp) return;
+    if (kind == 1 && absorb) return (q == 0 || q == 4) ? 1e-12 : 0.0;
+    if (kind == 1 && q >= 1 && q <= 3)
+    {
+        const double un = w[1] * n.x + w[2] * n.y + w[3] * n.z;
+        return w[q] - 2 * un * (q == 1 ? n.x : q == 2 ? n.y : n.z);
+    }
+    if (kind == 2) return q == 0 ? fs.rho : q == 1 ? fs.u : q == 2 ? fs.v : q == 3 ? fs.w : fs.p;
+    return w[q];
+}
+
+// K5: per (cell, species): the face-state transpose (lW, lG from the cell's four face slots), then the
+// reverse of the limited gradients.  lW holds the u+ part on entry and the cell's own total on exit;
+// slot[((s*4 + j)*5 + q)*nc + c] receives the adjoint of neighbour j's primitive q as this cell's stencil saw it.
+// blockDim = (32, 5) as k_limited_slots: warp q handles variable q of 32 cells with the stencil staged in shared memory.
+// The density and pressure warps tell the others which face states extrapolate; a wall or inflow ghost mixes the
+// variables, so the boundary slots' adjoints meet in shared memory and warp 0 takes them back.  second = 0: the forward
+// stage ran with zero gradients (every face state the cell's).
+// The limiter term that sets psi is the forward pass's: the quotient at the largest or the most negative dl, the first
+// face that has it, the earlier one where the two quotients tie.
+// 295k tetrahedra, two species: 170 us, 228 as one thread per (cell, species) (168 registers, spills).
+__global__ void __launch_bounds__(160, 4) k_a_grad(MeshView m, FluidParams p, int second, const double *__restrict__ W,
+                                                   const double *__restrict__ lface, double *__restrict__ lW, double *__restrict__ slot,
+                                                   double *__restrict__ lfs)
+{
+    constexpr int ROWS = 30;
+    __shared__ double geo[ROWS][32], sl[4][5][32], slw[5][32];
+    __shared__ uint32_t pos[2][4];
+    const int lane = threadIdx.x, q = threadIdx.y, s = blockIdx.x % p.nsp;
+    const int32_t c = (blockIdx.x / p.nsp) * 32 + lane;
     const int64_t n = m.nc, nf = m.nf;
-    double wc[5], g[15], lw[5], lG[15];
+    const bool in = c < m.nc, valid = in && c < m.no_cells && m.st_valid[c];
+    if (in)
 #pragma unroll
-    for (int q = 0; q < 5; ++q)
+        for (int r = 0; r < ROWS; r += 5) cp_async8(&geo[r + q][lane], m.t_wd + (r + q) * n + c);
+    cp_async_commit();
+    int32_t nb[4] = {INT32_MIN, INT32_MIN, INT32_MIN, INT32_MIN};
+    double lf[4], v[4], wc = 0, lw = 0, lwn[4] = {0, 0, 0, 0};
+    bool bnd = false;
+    if (in)
     {
-        wc[q] = W[ui(s, q, c, n)];
-        lw[q] = lW[ui(s, q, c, n)];
-    }
-#pragma unroll
-    for (int q = 0; q < 15; ++q)
-    {
-        g[q] = G[gi(s, q, c, n)];
-        lG[q] = 0.0;
-    }
-    const V3 xc = ld3(m.cell_center, c);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-    {
-        const int32_t f = m.c2f_idx[4 * c + j];
-        const int side = m.c2f_sgn[4 * c + j] > 0 ? 0 : 1;
-        double lf[5];
-        bool any = false;
-#pragma unroll
-        for (int q = 0; q < 5; ++q)
-        {
-            lf[q] = lface[((int64_t)(s * 2 + side) * 5 + q) * nf + f];
-            any |= lf[q] != 0.0;
-        }
-        if (!any) continue;
-        const V3 dx = ld3(m.face_center, f) - xc;
-        // face_state extrapolates unless the extrapolated density or pressure is not positive
-        const bool extrap = wc[0] + g[0] * dx.x + g[1] * dx.y + g[2] * dx.z > 0 && wc[4] + g[12] * dx.x + g[13] * dx.y + g[14] * dx.z > 0;
-#pragma unroll
-        for (int q = 0; q < 5; ++q)
-        {
-            lw[q] += lf[q];
-            if (extrap)
-            {
-                lG[3 * q] += lf[q] * dx.x;
-                lG[3 * q + 1] += lf[q] * dx.y;
-                lG[3 * q + 2] += lf[q] * dx.z;
-            }
-        }
-    }
-    double lwn[4][5];
-    int32_t nb[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-    {
-        nb[j] = m.t_nb[j * n + c];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) lwn[j][q] = 0.0;
-    }
-    const bool valid = c < m.no_cells && m.st_valid[c];
-    if (valid)
-    {
-        const Prim5 wcp{wc[0], wc[1], wc[2], wc[3], wc[4]};
-        double wn[4][5], wd[12], dxs[12];
+        const double *w = W + ui(s, q, 0, n);
+        wc = w[c];
+        lw = lW[ui(s, q, c, n)];
+        const int4 fi = *reinterpret_cast<const int4 *>(m.c2f_idx + 4 * (int64_t)c);
+        const char4 sg = *reinterpret_cast<const char4 *>(m.c2f_sgn + 4 * (int64_t)c);
+        const int32_t ff[4] = {fi.x, fi.y, fi.z, fi.w};
+        const bool out[4] = {sg.x > 0, sg.y > 0, sg.z > 0, sg.w > 0};
 #pragma unroll
         for (int j = 0; j < 4; ++j)
         {
-            if (nb[j] >= 0)
-            {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) wn[j][q] = W[ui(s, q, nb[j], n)];
-            }
-            else if (nb[j] != INT32_MIN)
-            {
-                const int32_t f = -(nb[j] + 1);
-                const V3 nrm = (double(m.t_sg[j * n + c]) / m.face_area_mag[f]) * ld3(m.face_area, f);
-                const Prim5 gh = ghost_state(m.face_kind[f], p.absorb[s] != 0, wcp, nrm, p.fs[s]);
-                wn[j][0] = gh.rho; wn[j][1] = gh.u; wn[j][2] = gh.v; wn[j][3] = gh.w; wn[j][4] = gh.p;
-            }
-            else
-            {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) wn[j][q] = 0.0;
-            }
+            lf[j] = lface[((int64_t)(s * 2 + (out[j] ? 0 : 1)) * 5 + q) * nf + ff[j]];
+            nb[j] = m.t_nb[j * n + c];
+            bnd |= valid && nb[j] < 0 && nb[j] != INT32_MIN;
         }
 #pragma unroll
-        for (int i = 0; i < 12; ++i)
+        for (int j = 0; j < 4; ++j) v[j] = nb[j] >= 0 ? w[nb[j]] : wc;
+        if (bnd)
         {
-            wd[i] = m.t_wd[i * n + c];
-            dxs[i] = m.t_dx[i * n + c];
-        }
-        const double I00 = m.t_inv[c], I01 = m.t_inv[n + c], I02 = m.t_inv[2 * n + c], I11 = m.t_inv[3 * n + c],
-                     I12 = m.t_inv[4 * n + c], I22 = m.t_inv[5 * n + c];
-#pragma unroll
-        for (int q = 0; q < 5; ++q)
-        {
-            if (lG[3 * q] == 0.0 && lG[3 * q + 1] == 0.0 && lG[3 * q + 2] == 0.0) continue;
-            double r0 = 0, r1 = 0, r2 = 0, lo = wc[q], hi = wc[q];
-            int jlo = -1, jhi = -1;
-#pragma unroll
+            const double wv[5] = {W[ui(s, 0, c, n)], W[ui(s, 1, c, n)], W[ui(s, 2, c, n)], W[ui(s, 3, c, n)], W[ui(s, 4, c, n)]};
             for (int j = 0; j < 4; ++j)
             {
-                if (nb[j] == INT32_MIN) continue;
-                const double dq = wn[j][q] - wc[q];
-                r0 += wd[3 * j] * dq;
-                r1 += wd[3 * j + 1] * dq;
-                r2 += wd[3 * j + 2] * dq;
-                if (wn[j][q] < lo)
-                {
-                    lo = wn[j][q];
-                    jlo = j;
-                }
-                if (hi < wn[j][q])
-                {
-                    hi = wn[j][q];
-                    jhi = j;
-                }
+                const int32_t b = m.t_nb[j * n + c];
+                if (b >= 0 || b == INT32_MIN) continue;
+                const D4 fn = ld_d4(m.fna + 4 * (int64_t)(-(b + 1)));
+                const double t = m.t_sg[j * n + c];
+                const double g = ghost_q(m.face_kind[-(b + 1)], p.absorb[s] != 0, q, wv, mk(t * fn.x, t * fn.y, t * fn.z), p.fs[s]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k == j) v[k] = g;
             }
-            const double g0 = I00 * r0 + I01 * r1 + I02 * r2;
-            const double g1 = I01 * r0 + I11 * r1 + I12 * r2;
-            const double g2 = I02 * r0 + I12 * r1 + I22 * r2;
-            double psi = 1.0, wdl = 0, wx = 0, wy = 0, wz = 0;
-            int wtype = -1; // the limiter term that set psi: 0 hi, 1 lo, 2 relative
-            if (p.limit)
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) lw += lf[j];
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    const double(*dx)[32] = geo + 12;
+    double lo = wc, hi = wc, g0 = 0, g1 = 0, g2 = 0, dpos = 0, dneg = 0, psi = 1.0;
+    int jlo = -1, jhi = -1, jpos = 0, jneg = 0, wtype = -1; // wtype: the limiter term that set psi: 0 hi, 1 lo, 2 relative
+    double I00, I01, I02, I11, I12, I22;
+    auto limit = [&] {
+        if (!p.limit) return;
+        const double n1 = hi - wc, n2 = lo - wc;
+        const bool c1 = dpos > 1e-300 && n1 < dpos, c2 = dneg < -1e-300 && n2 > dneg;
+        if (c1 || c2)
+        {
+            bool first = c1;
+            if (c1 && c2)
             {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
+                const double p1 = n1 * -dneg, p2 = -n2 * dpos;
+                first = p1 < p2;
+                if (p1 == p2)
                 {
-                    const double d = g0 * dxs[3 * j] + g1 * dxs[3 * j + 1] + g2 * dxs[3 * j + 2];
-                    double x = psi;
-                    int ty = -1;
-                    if (d > 1e-300) { x = (hi - wc[q]) / d; ty = 0; }
-                    else if (d < -1e-300) { x = (lo - wc[q]) / d; ty = 1; }
-                    if (ty >= 0 && x < psi)
-                    {
-                        psi = x; wtype = ty; wdl = d;
-                        wx = dxs[3 * j]; wy = dxs[3 * j + 1]; wz = dxs[3 * j + 2];
-                    }
+                    const double x0 = n1 / dpos, x1 = n2 / dneg;
+                    first = x0 < x1 || (x0 == x1 && jpos < jneg);
                 }
-                if (p.rel_limit > 0 && (q == 0 || q == 4))
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                    {
-                        const double d = g0 * dxs[3 * j] + g1 * dxs[3 * j + 1] + g2 * dxs[3 * j + 2];
-                        const double da = fabs(d);
-                        if (da > 1e-300)
-                        {
-                            const double x = p.rel_limit * wc[q] / da;
-                            if (x < psi)
-                            {
-                                psi = x; wtype = 2; wdl = d;
-                                wx = dxs[3 * j]; wy = dxs[3 * j + 1]; wz = dxs[3 * j + 2];
-                            }
-                        }
-                    }
             }
+            const double num = first ? n1 : n2;
+            psi = num == 0 ? 0.0 : num / (first ? dpos : dneg);
+            wtype = first ? 0 : 1;
+        }
+        if (p.rel_limit > 0 && (q == 0 || q == 4))
+        {
+            const double a = dmax(dpos, -dneg);
+            if (a > 1e-300)
+            {
+                const double x = p.rel_limit * wc / a;
+                if (x < psi)
+                {
+                    psi = x;
+                    wtype = 2;
+                }
+            }
+        }
+    };
+    if (valid)
+    {
+        double r0 = 0, r1 = 0, r2 = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const double dq = v[j] - wc;
+            r0 += geo[3 * j][lane] * dq;
+            r1 += geo[3 * j + 1][lane] * dq;
+            r2 += geo[3 * j + 2][lane] * dq;
+            if (v[j] < lo)
+            {
+                lo = v[j];
+                jlo = j;
+            }
+            if (hi < v[j])
+            {
+                hi = v[j];
+                jhi = j;
+            }
+        }
+        I00 = geo[24][lane]; I01 = geo[25][lane]; I02 = geo[26][lane]; I11 = geo[27][lane]; I12 = geo[28][lane]; I22 = geo[29][lane];
+        g0 = I00 * r0 + I01 * r1 + I02 * r2;
+        g1 = I01 * r0 + I11 * r1 + I12 * r2;
+        g2 = I02 * r0 + I12 * r1 + I22 * r2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const double d = g0 * dx[3 * j][lane] + g1 * dx[3 * j + 1][lane] + g2 * dx[3 * j + 2][lane];
+            if (d > dpos)
+            {
+                dpos = d;
+                jpos = j;
+            }
+            if (d < dneg)
+            {
+                dneg = d;
+                jneg = j;
+            }
+        }
+    }
+    // face_state extrapolates unless the extrapolated density or pressure is not positive
+    if (q == 0 || q == 4)
+    {
+        double G0 = 0, G1 = 0, G2 = 0;
+        if (valid)
+        {
+            limit();
+            const double ps = second ? dmax(0.0, dmin(1.0, psi)) : 0.0;
+            G0 = ps * g0;
+            G1 = ps * g1;
+            G2 = ps * g2;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const bool up = valid && wc + G0 * dx[3 * j][lane] + G1 * dx[3 * j + 1][lane] + G2 * dx[3 * j + 2][lane] > 0;
+            const uint32_t b = __ballot_sync(0xffffffffu, up);
+            if (lane == 0) pos[q >> 2][j] = b;
+        }
+    }
+    __syncthreads();
+    if (valid)
+    {
+        double lG0 = 0, lG1 = 0, lG2 = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((pos[0][j] & pos[1][j]) >> lane & 1u)
+            {
+                lG0 += lf[j] * dx[3 * j][lane];
+                lG1 += lf[j] * dx[3 * j + 1][lane];
+                lG2 += lf[j] * dx[3 * j + 2][lane];
+            }
+        if (lG0 != 0.0 || lG1 != 0.0 || lG2 != 0.0)
+        {
+            if (q != 0 && q != 4) limit();
             const double ps = dmax(0.0, dmin(1.0, psi));
-            double lg0 = ps * lG[3 * q], lg1 = ps * lG[3 * q + 1], lg2 = ps * lG[3 * q + 2];
-            double lwc = 0, lhi = 0, llo = 0;
+            double lg0 = ps * lG0, lg1 = ps * lG1, lg2 = ps * lG2, lwc = 0, lhi = 0, llo = 0;
             if (psi < 1.0 && 0.0 < psi && wtype >= 0)
             {
-                const double lpsi = lG[3 * q] * g0 + lG[3 * q + 1] * g1 + lG[3 * q + 2] * g2;
+                const double lpsi = lG0 * g0 + lG1 * g1 + lG2 * g2;
+                // the winning face: the relative limiter's is the first with the largest |dl|
+                const bool up = wtype == 2 ? (dpos > -dneg || (dpos == -dneg && jpos < jneg)) : wtype == 0;
+                const double wdl = up ? dpos : dneg;
+                const int wj = up ? jpos : jneg;
                 double ldl;
                 if (wtype == 2)
                 {
@@ -1265,14 +1283,15 @@ __global__ void __launch_bounds__(128, 3) k_a_grad(MeshView m, FluidParams p, co
                 }
                 else
                 {
-                    if (wtype == 0) lhi += lpsi / wdl;
-                    else llo += lpsi / wdl;
-                    lwc -= lpsi / wdl;
+                    const double t = lpsi / wdl;
+                    if (wtype == 0) lhi += t;
+                    else llo += t;
+                    lwc -= t;
                     ldl = -psi * lpsi / wdl;
                 }
-                lg0 += ldl * wx;
-                lg1 += ldl * wy;
-                lg2 += ldl * wz;
+                lg0 += ldl * dx[3 * wj][lane];
+                lg1 += ldl * dx[3 * wj + 1][lane];
+                lg2 += ldl * dx[3 * wj + 2][lane];
             }
             if (jhi < 0) lwc += lhi;
             if (jlo < 0) lwc += llo;
@@ -1285,29 +1304,41 @@ __global__ void __launch_bounds__(128, 3) k_a_grad(MeshView m, FluidParams p, co
                 double a = (j == jhi ? lhi : 0.0) + (j == jlo ? llo : 0.0);
                 if (nb[j] != INT32_MIN)
                 {
-                    const double d = wd[3 * j] * lr0 + wd[3 * j + 1] * lr1 + wd[3 * j + 2] * lr2;
+                    const double d = geo[3 * j][lane] * lr0 + geo[3 * j + 1][lane] * lr1 + geo[3 * j + 2][lane] * lr2;
                     a += d;
                     lwc -= d;
                 }
-                lwn[j][q] += a;
+                lwn[j] = a;
             }
-            lw[q] += lwc;
+            lw += lwc;
         }
+        if (bnd)
+        {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (nb[j] < 0 && nb[j] != INT32_MIN)
-            {
-                const int32_t f = -(nb[j] + 1);
-                const V3 nrm = (double(m.t_sg[j * n + c]) / m.face_area_mag[f]) * ld3(m.face_area, f);
-                ghost_T(m.face_kind[f], p.absorb[s] != 0, nrm, lwn[j], lw, lfs + 5 * s);
-            }
+            for (int j = 0; j < 4; ++j) sl[j][q][lane] = lwn[j];
+            slw[q][lane] = lw;
+        }
     }
+    if (in)
+    {
 #pragma unroll
+        for (int j = 0; j < 4; ++j) slot[((int64_t)(s * 4 + j) * 5 + q) * n + c] = nb[j] >= 0 ? lwn[j] : 0.0;
+        if (!bnd) lW[ui(s, q, c, n)] = lw;
+    }
+    if (!__syncthreads_or(bnd) || q != 0 || !bnd) return;
+    double t[5];
+    for (int k = 0; k < 5; ++k) t[k] = slw[k][lane];
     for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int q = 0; q < 5; ++q) slot[((int64_t)(s * 4 + j) * 5 + q) * n + c] = nb[j] >= 0 ? lwn[j][q] : 0.0;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) lW[ui(s, q, c, n)] = lw[q];
+    {
+        const int32_t b = m.t_nb[j * n + c];
+        if (b >= 0 || b == INT32_MIN) continue;
+        const int32_t f = -(b + 1);
+        const D4 fn = ld_d4(m.fna + 4 * (int64_t)f);
+        const double sg = m.t_sg[j * n + c];
+        const double lg[5] = {sl[j][0][lane], sl[j][1][lane], sl[j][2][lane], sl[j][3][lane], sl[j][4][lane]};
+        ghost_T(m.face_kind[f], p.absorb[s] != 0, mk(sg * fn.x, sg * fn.y, sg * fn.z), lg, t, lfs + 5 * s);
+    }
+    for (int k = 0; k < 5; ++k) lW[ui(s, k, c, n)] = t[k];
 }
 
 // K6: per cell: lW + the neighbours' stencil slots pointing here (rslot: the slot of neighbour j that holds
@@ -1441,7 +1472,7 @@ struct MhdFn
     // a stage's primitives, limited gradients and cell fields, as the stage left them in the state's buffers
     struct StageFields
     {
-        DBuf<double> W, G, up, bind, btot;
+        DBuf<double> W, FV, up, bind, btot;
     };
     struct TapeStep
     {
@@ -1684,14 +1715,14 @@ void adjoint_stage(MhdFn *fn, const double *Uin, const double *Pin, const double
     if (m.nf)
     {
         P.begin(FN_ADJ_FLUX, s);
-        k_a_flux<<<dim3(g128(m.nf), nsp), 128, 0, s>>>(m, st->fp, st->W.p, st->grad.p, fn->lrV.p, fn->lface.p, fn->lpar.p + 3, fn->y.p,
-                                                        lPin);
+        k_a_flux<<<g128(m.nf) * nsp, 128, 0, s>>>(m, st->fp, st->fv.p, fn->lrV.p, fn->lface.p, fn->lpar.p + 3, fn->y.p, lPin);
         P.end(FN_ADJ_FLUX, s);
     }
     if (nc)
     {
         P.begin(FN_ADJ_GRAD, s);
-        k_a_grad<<<dim3(g128(nc), nsp), 128, 0, s>>>(m, st->fp, st->W.p, st->grad.p, fn->lface.p, fn->lW.p, fn->slot.p, fn->lpar.p + 3);
+        k_a_grad<<<grid_for(nc, 32) * nsp, dim3(32, 5), 0, s>>>(m, st->fp, st->prm.second_order, st->W.p, fn->lface.p, fn->lW.p, fn->slot.p,
+                                                               fn->lpar.p + 3);
         P.end(FN_ADJ_GRAD, s);
         P.begin(FN_ADJ_PRIM, s);
         k_a_prim<<<dim3(g128(nc), nsp), 128, 0, s>>>(m, st->fp, Uin, fn->lW.p, fn->slot.p, fn->rslot.p, lUin);
@@ -1704,7 +1735,7 @@ void adjoint_stage(MhdFn *fn, const double *Uin, const double *Pin, const double
 void swap_fields(MhdState *st, MhdFn::StageFields &f)
 {
     std::swap(st->W.p, f.W.p);
-    std::swap(st->grad.p, f.G.p);
+    std::swap(st->fv.p, f.FV.p);
     std::swap(st->up.p, f.up.p);
     std::swap(st->bind.p, f.bind.p);
     std::swap(st->btot.p, f.btot.p);
@@ -1718,7 +1749,7 @@ void alloc_step(MhdFn *fn, MhdFn::TapeStep &T)
     T.fl1.alloc(fn->nsp * nc); T.fl2.alloc(fn->nsp * nc);
     for (auto &f : T.sf)
     {
-        f.W.alloc(fn->st->W.n); f.G.alloc(fn->st->grad.n); f.up.alloc(3 * nc); f.bind.alloc(3 * nc); f.btot.alloc(3 * nc);
+        f.W.alloc(fn->st->W.n); f.FV.alloc(fn->st->fv.n); f.up.alloc(3 * nc); f.bind.alloc(3 * nc); f.btot.alloc(3 * nc);
     }
 }
 
@@ -1791,6 +1822,7 @@ void alloc_tangent(MhdFn *fn)
         fn->tU[i].alloc(5 * ns * nc); fn->dU[i].alloc(5 * ns * nc);
         fn->tP[i].alloc(nf); fn->dP[i].alloc(nf);
     }
+    fn->st->grad.alloc(15 * ns * nc);
     fn->dW.alloc(5 * ns * nc); fn->dG.alloc(15 * ns * nc); fn->dF.alloc(5 * ns * nf);
     fn->dup.alloc(3 * nc); fn->dbi.alloc(3 * nc); fn->dbt.alloc(3 * nc); fn->dEf.alloc(3 * nf); fn->dE.alloc(ne);
     fn->dm.alloc(ne); fn->deta.alloc(nc);
@@ -1866,7 +1898,6 @@ int mhd_gpu_fn_create(MhdState *st, const MhdFnParams *p, const double *eta, con
         fn->X0P.alloc(nf);
         copy_d(fn->X0U.p, st->U0.p, 5 * fn->nsp * nc, s);
         copy_d(fn->X0P.p, st->phi0.p, nf, s);
-        st->grad.alloc(15 * nc * st->group); // the recorded stages and the tangent run keep the gradients
         st->mres.alloc(ne);
         fn->active.alloc(nf);
         fn->rslot.alloc(4 * nc);
@@ -1940,6 +1971,7 @@ struct SwitchScope
         MhdState *st = fn->st;
         for (auto &b : fn->sw)
             if (b.n) MHD_CUDA(cudaMemsetAsync(b.p, 0, b.n * sizeof(uint32_t), stream_of(fn)));
+        st->grad.alloc(15 * (size_t)st->mesh->v.nc * fn->nsp); // the logging passes go through the gradients
         st->fp.sw_lim = fn->sw[0].p;
         st->fp.sw_flux = fn->sw[1].p;
         st->sw_edge = fn->sw[2].p;

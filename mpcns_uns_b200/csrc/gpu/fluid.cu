@@ -539,12 +539,30 @@ void launch_limited_gradients(const MeshView &m, const FluidParams &p, SField<co
     MHD_LAUNCH_CHECK();
 }
 
-void launch_face_values(const MeshView &m, const FluidParams &p, SField<const double> W, const SField<double> *G, double *FV, cudaStream_t s)
+// the face values of the first-order scheme: every face the cell's value
+template <int NF>
+__global__ void __launch_bounds__(128) k_cell_face_values(int32_t nc, int nrow, const double *__restrict__ W, double *__restrict__ FV)
+{
+    pdl_begin();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; // (species, variable) row and cell
+    if (i >= (int64_t)nrow * nc) return;
+    const double w = W[i];
+    for (int j = 0; j < NF; ++j) FV[i * NF + j] = w;
+}
+
+void launch_face_values(const MeshView &m, const FluidParams &p, SField<const double> W, bool second_order, const SField<double> *G,
+                        double *FV, cudaStream_t s)
 {
     if (!m.nc) return;
-    const SField<double> g0 = G ? *G : SField<double>{};
-    if (m.faces_per_cell == 4) (G ? launch_slots<4, false, true, true> : launch_slots<4, false, false, true>)(m, p, W, g0, FV, s);
-    else (G ? launch_slots<6, false, true, true> : launch_slots<6, false, false, true>)(m, p, W, g0, FV, s);
+    if (!second_order)
+    {
+        const int64_t rows = 5 * p.nsp;
+        launch_pdl(m.faces_per_cell == 4 ? k_cell_face_values<4> : k_cell_face_values<6>, grid_for(rows * m.nc, 128), 128, 0, s, m.nc,
+                   static_cast<int>(rows), W.p, FV);
+    }
+    else if (m.faces_per_cell == 6) launch_slots<6, false, false, true>(m, p, W, SField<double>{}, FV, s);
+    else if (G) launch_slots<4, true, true, true>(m, p, W, *G, FV, s);
+    else launch_slots<4, false, false, true>(m, p, W, SField<double>{}, FV, s);
     MHD_LAUNCH_CHECK();
 }
 

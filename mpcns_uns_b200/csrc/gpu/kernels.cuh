@@ -11,9 +11,11 @@ MhdMesh *induction_mesh(const MhdInduction *I);
 // fluid.cu
 void launch_limited_gradients(const MeshView &m, const FluidParams &p, SField<const double> W, SField<double> G, cudaStream_t s);
 void launch_face_flux(const MeshView &m, const FluidParams &p, SField<const double> W, SField<const double> G, double *F, cudaStream_t s);
-// limited face values of every cell (meshes with faces_per_cell > 0; FV holds 5 * faces_per_cell * nc values per species),
-// with G also the limited gradients; the face flux from them
-void launch_face_values(const MeshView &m, const FluidParams &p, SField<const double> W, const SField<double> *G, double *FV, cudaStream_t s);
+// limited face values of every cell (meshes with faces_per_cell > 0; FV holds 5 * faces_per_cell * nc values per species;
+// the cell's own values unless second_order), with G (tetrahedra, second order) also the limited gradients and the switch
+// log; the face flux from them
+void launch_face_values(const MeshView &m, const FluidParams &p, SField<const double> W, bool second_order, const SField<double> *G,
+                        double *FV, cudaStream_t s);
 void launch_face_flux_fv(const MeshView &m, const FluidParams &p, const double *FV, double *F, cudaStream_t s);
 
 // induction.cu

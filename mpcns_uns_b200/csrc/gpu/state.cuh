@@ -45,7 +45,7 @@ struct MhdState
     mhd::FluidParams fp{};
     int nsp = 0, group = 0;
     bool mixed = false;
-    mhd::DBuf<double> fv; // FP64 second-order state on a mesh of one cell kind: limited face values (launch_face_values)
+    mhd::DBuf<double> fv; // FP64 state on a mesh of one cell kind: face values (launch_face_values); others keep grad
     mhd::DBuf<double> U0, U1, W, grad, F, phi0, phi1, phi_add, badd, bind, btot, up, Ef, E, mass, stage;
     mhd::SrcParams src;     // two-ion J x B force and gyration (off unless params.lorentz)
     mhd::DBuf<double> J;    // cell current of the induced field (3 per cell) when the J x B force is on
@@ -145,8 +145,6 @@ __device__ __forceinline__ void cfl_reduce(const CflOut &o, double v, bool bad)
 void mixed_setup(MhdState *st);
 // one FP64 stage (Us, phis) -> (Uo, phio) at the step size in st->scal[0]; stage2 averages with Uo, phio in place
 void fp64_stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2);
-// its first half alone: primitives, cell fields, u+ and limited gradients of (Us, phis) into st's buffers
-void fp64_prepare_grad(MhdState *st, const double *Us, const double *phis);
 // gyrate_close: stage 2 applies the closing half-step gyration in its update (two-ion sources on)
 void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2, bool cfl, double dt_max,
                  bool prepared = false, bool gyrate_close = false);

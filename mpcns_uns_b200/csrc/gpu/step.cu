@@ -379,13 +379,19 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
         if (gp.sw_flux) gp.sw_flux += (int64_t)s0 * m.nf;
         const SField<const double> Wg{st->W.p + (int64_t)s0 * 5 * nc, 5 * nc, 1, nc};
         const SField<double> Gg{st->grad.p, 15 * nc, 1, nc};
-        // face values where the state holds them, with the gradients too while a differentiated run records its
-        // stages (floor_flags); the gradients alone for the first-order scheme, mixed polyhedra and the switch log
-        const bool faces = st->fv.n && !gp.sw_lim && !gp.sw_flux;
+        // face values where the state holds them; with the switch log on the fluxes come from the gradients, which tell
+        // the limiter's and the face states' choices, and a recorded stage (floor_flags) gets its face values as well
+        const bool log = gp.sw_lim || gp.sw_flux, faces = st->fv.n && !log;
         P.begin(KP_GRAD, s);
-        if (faces) launch_face_values(m, gp, Wg, st->floor_flags ? &Gg : nullptr, st->fv.p, s);
-        else if (st->prm.second_order) launch_limited_gradients(m, gp, Wg, Gg, s);
-        else MHD_CUDA(cudaMemsetAsync(st->grad.p, 0, (size_t)15 * ng * nc * sizeof(double), s));
+        if (faces) launch_face_values(m, gp, Wg, st->prm.second_order, nullptr, st->fv.p, s);
+        else if (st->prm.second_order && st->fv.n && gp.sw_lim && st->floor_flags)
+            launch_face_values(m, gp, Wg, true, &Gg, st->fv.p, s);
+        else
+        {
+            if (st->prm.second_order) launch_limited_gradients(m, gp, Wg, Gg, s);
+            else MHD_CUDA(cudaMemsetAsync(st->grad.p, 0, (size_t)15 * ng * nc * sizeof(double), s));
+            if (log && st->fv.n && st->floor_flags) launch_face_values(m, gp, Wg, false, nullptr, st->fv.p, s);
+        }
         P.end(KP_GRAD, s);
         P.begin(KP_FLUX, s);
         if (faces) launch_face_flux_fv(m, gp, st->fv.p, st->F.p, s);
@@ -442,20 +448,6 @@ void cfl_empty(MhdState *st, double dt_max)
 void fp64_stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2)
 {
     stage(st, Us, phis, Uo, phio, stage2, false, 0.0);
-}
-
-// The first half of a stage: primitives, cell fields, u+ and the limited gradients of every species
-// (one species group) of (Us, phis), as fp64_stage leaves them
-void fp64_prepare_grad(MhdState *st, const double *Us, const double *phis)
-{
-    MHD_REQUIRE(st->nsp <= st->group, "one species group");
-    prepare_cfl(st, Us, phis, false, 0.0);
-    const MeshView &m = st->mesh->v;
-    const int64_t nc = m.nc;
-    const SField<const double> Wg{st->W.p, 5 * nc, 1, nc};
-    const SField<double> Gg{st->grad.p, 15 * nc, 1, nc};
-    if (st->prm.second_order) launch_limited_gradients(m, st->fp, Wg, Gg, st->mesh->stream);
-    else if (nc) MHD_CUDA(cudaMemsetAsync(st->grad.p, 0, (size_t)15 * st->nsp * nc * sizeof(double), st->mesh->stream));
 }
 
 namespace
@@ -546,7 +538,7 @@ int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *p, MhdState **out)
         st->W.alloc(5 * nc * st->nsp);
         if (p->precision != MHD_PREC_MIXED)
         {
-            if (p->second_order && m.faces_per_cell) st->fv.alloc(5 * (size_t)m.faces_per_cell * nc * st->group);
+            if (m.faces_per_cell) st->fv.alloc(5 * (size_t)m.faces_per_cell * nc * st->group);
             else st->grad.alloc(15 * nc * st->group);
             st->F.alloc(5 * nf * st->group);
         }

@@ -122,36 +122,4 @@ __device__ __forceinline__ DV3 cell_vector_d(const MeshView &m, DCPtr flux, int3
     return dmk(I[0][0] * r[0] + I[0][1] * r[1] + I[0][2] * r[2], I[1][0] * r[0] + I[1][1] * r[1] + I[1][2] * r[2],
                I[2][0] * r[0] + I[2][1] * r[1] + I[2][2] * r[2]);
 }
-
-// The inverse normal matrix of uns::reconstruct_cell_vector: B_c = I_c sum_k n_k phi_k (n_k the face's
-// unit normal as stored, phi_k its flux).  Returns false where the reference returns a zero vector.
-__device__ __forceinline__ bool cell_vector_inverse(const MeshView &m, int32_t c, double I[3][3])
-{
-    double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int32_t k = m.c2f_ptr[c]; k < m.c2f_ptr[c + 1]; ++k)
-    {
-        const int32_t f = m.c2f_idx[k];
-        const double A = m.face_area_mag[f];
-        if (A <= 0) continue;
-        const double s = m.c2f_sgn[k];
-        const V3 n = (s / A) * ld3(m.face_area, f);
-        const double nv[3] = {n.x, n.y, n.z};
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) M[i][j] += A * nv[i] * nv[j];
-    }
-    const double det = M[0][0] * (M[1][1] * M[2][2] - M[1][2] * M[2][1]) - M[0][1] * (M[1][0] * M[2][2] - M[1][2] * M[2][0]) +
-                       M[0][2] * (M[1][0] * M[2][1] - M[1][1] * M[2][0]);
-    const double sc = dmax(dmax(dmax(M[0][0], M[1][1]), M[2][2]), 1e-300);
-    if (fabs(det) < 1e-12 * sc * sc * sc) return false;
-    I[0][0] = (M[1][1] * M[2][2] - M[1][2] * M[2][1]) / det;
-    I[0][1] = (M[0][2] * M[2][1] - M[0][1] * M[2][2]) / det;
-    I[0][2] = (M[0][1] * M[1][2] - M[0][2] * M[1][1]) / det;
-    I[1][0] = (M[1][2] * M[2][0] - M[1][0] * M[2][2]) / det;
-    I[1][1] = (M[0][0] * M[2][2] - M[0][2] * M[2][0]) / det;
-    I[1][2] = (M[0][2] * M[1][0] - M[0][0] * M[1][2]) / det;
-    I[2][0] = (M[1][0] * M[2][1] - M[1][1] * M[2][0]) / det;
-    I[2][1] = (M[0][1] * M[2][0] - M[0][0] * M[2][1]) / det;
-    I[2][2] = (M[0][0] * M[1][1] - M[0][1] * M[1][0]) / det;
-    return true;
-}
 } // namespace mhd
