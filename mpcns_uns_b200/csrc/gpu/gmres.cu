@@ -23,8 +23,8 @@
 //     tail of w and V_{i-1} left in L2 is reused first;
 //   * every dot of the operator finishes in the kernel that produces it (the last block adds the block partials), those
 //     of Gram-Schmidt in k_cgs_tail, which also rotates the column, and
-//     a restart cycle runs as one CUDA graph whose steps test a device-side flag, so the host waits
-//     once per restart instead of once per Arnoldi step.
+//     a restart cycle runs as CUDA graphs of a few steps whose kernels test a device-side flag, so the host does not
+//     wait for the device within a restart.
 #include <array>
 #include <utility>
 
@@ -288,10 +288,12 @@ __global__ void k_vec_v0(int32_t n, const double *r, const double *beta, double 
 }
 
 // start of a restart cycle: g = (beta, 0, ...), at most `limit` Arnoldi steps, early exit at |g_{j+1}| <= tol
-__global__ void k_cycle_init(Ctl *ctl, int limit, double tol, double dt, double *g, int n, const double *beta)
+__global__ void k_cycle_init(Ctl *ctl, int limit, double tol, double dt, double *g, int n, const double *beta, int *host_done)
 {
     pdl_begin();
     ctl->done = 0;
+    ctl->host_done = host_done;
+    *host_done = 0;
     ctl->jend = 0;
     ctl->limit = limit;
     ctl->reorth = 0;
@@ -323,7 +325,11 @@ __global__ void k_givens(Ctl *ctl, double *H, int mcols, int j, double *cs, doub
     g[j + 1] = -sn[j] * g[j];
     g[j] = cs[j] * g[j];
     ctl->jend = j + 1;
-    if (fabs(g[j + 1]) <= ctl->tol) ctl->done = 1;
+    if (fabs(g[j + 1]) <= ctl->tol)
+    {
+        ctl->done = 1;
+        *ctl->host_done = 1;
+    }
 }
 
 // The sums of a Gram-Schmidt pass from its blocks' rows of partial sums, and what they decide.
@@ -409,7 +415,11 @@ __global__ void __launch_bounds__(512) k_cgs_tail(Gate gt, Ctl *ctl, int pass, i
     g[j] = cs * gj;
     ctl->jend = j + 1;
     ctl->reorth = 0;
-    if (fabs(gn) <= ctl->tol) ctl->done = 1;
+    if (fabs(gn) <= ctl->tol)
+    {
+        ctl->done = 1;
+        *ctl->host_done = 1;
+    }
 }
 
 // The back substitution below for at most 32 steps by one warp: lane i holds row i and forms its product with every y_k as
@@ -577,17 +587,17 @@ void dev_dot(MhdInduction *I, const double *a, const double *b, int op, double *
     IND_LAUNCH(I, KI_VECTOR, s, launch_pdl(k_dot, kRedBlocks, 256, 0, s, a, b, I->mesh->v.no_edges, I->part.p, I->counter.p, op, out));
 }
 
-// The mr Arnoldi steps of one restart cycle (:333-348), each gated by the cycle control:
+// Arnoldi steps j0 to j1 - 1 of one restart cycle (:333-348), each gated by the cycle control:
 // w = A P^-1 V_j with V_j = w_prev / H(j, j-1) formed on the fly, Dirichlet rows zeroed and H(0, j) = w . V_0;
 // modified Gram-Schmidt w -= H(i-1, j) V_{i-1} fused with H(i, j) = w . V_i; Givens and the early-exit test.
-void enqueue_cycle(MhdInduction *I)
+void enqueue_cycle(MhdInduction *I, int j0, int j1)
 {
     const MeshView &m = I->mesh->v;
     cudaStream_t s = I->mesh->stream;
     const int32_t ne = m.ne;
     const int mr = I->p.restart;
     double *V = I->V.p, *H = I->H.p;
-    for (int j = 0; j < mr; ++j)
+    for (int j = j0; j < j1; ++j)
     {
         Gate gt;
         gt.ctl = I->ctl.p;
@@ -647,40 +657,70 @@ void enqueue_cycle(MhdInduction *I)
     }
 }
 
-// Capture the cycle once as a CUDA graph; a stream that cannot be captured keeps direct launches.
-void build_cycle_graph(MhdInduction *I)
+// Capture the cycle's chunks once as CUDA graphs; a stream that cannot be captured keeps direct launches.
+void build_cycle_graphs(MhdInduction *I)
 {
-    const int md = I->mode;
+    const int md = I->mode, mr = I->p.restart;
     I->cycle_tried[md] = true;
     cudaStream_t s = I->mesh->stream;
-    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+    std::vector<MhdInduction::Chunk> chunks;
+    bool ok = true;
+    for (int j0 = 0; j0 < mr && ok; j0 += kCycleChunk)
     {
-        cudaGetLastError();
-        return;
-    }
-    const int64_t l0 = I->launches;
-    I->capturing = true;
-    enqueue_cycle(I);
-    I->capturing = false;
-    cudaGraph_t graph = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(s, &graph);
-    I->cycle_kernels[md] = I->launches - l0;
-    I->launches = l0;
-    if (ce != cudaSuccess || !graph)
-    {
-        cudaGetLastError();
+        ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+        if (!ok) break;
+        const int64_t l0 = I->launches;
+        I->capturing = true;
+        enqueue_cycle(I, j0, std::min(mr, j0 + kCycleChunk));
+        I->capturing = false;
+        cudaGraph_t graph = nullptr;
+        MhdInduction::Chunk c;
+        ok = cudaStreamEndCapture(s, &graph) == cudaSuccess && graph;
+        c.kernels = I->launches - l0;
+        I->launches = l0;
+        ok = ok && cudaGraphInstantiate(&c.exec, graph, 0) == cudaSuccess;
         if (graph) cudaGraphDestroy(graph);
-        return;
+        if (ok) chunks.push_back(c);
     }
-    cudaGraphExec_t exec = nullptr;
-    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ie != cudaSuccess)
+    if (ok) I->cycle[md] = std::move(chunks);
+    else
     {
         cudaGetLastError();
-        return;
+        for (auto &c : chunks) cudaGraphExecDestroy(c.exec);
     }
-    I->cycle[md] = exec;
+}
+
+// The cycle's steps up to limit: chunk k is launched when chunk k - 2 has finished without meeting the tolerance, so that
+// the device always has a chunk queued.
+void run_cycle(MhdInduction *I, int limit)
+{
+    const int mr = I->p.restart, steps = std::min(mr, limit);
+    cudaStream_t s = I->mesh->stream;
+    if (!I->prof.on && !I->cycle_tried[I->mode]) build_cycle_graphs(I);
+    const auto &chunks = I->cycle[I->mode];
+    const volatile int *done = reinterpret_cast<const int *>(I->pinned + 7);
+    for (int k = 0; k * kCycleChunk < steps; ++k)
+    {
+        if (k >= 2)
+        {
+            MHD_CUDA(cudaEventSynchronize(I->chunk_done[k - 2]));
+            if (*done) break;
+        }
+        if (!I->prof.on && !chunks.empty())
+        {
+            MHD_CUDA(cudaGraphLaunch(chunks[k].exec, s));
+            I->launches += chunks[k].kernels;
+        }
+        else
+            enqueue_cycle(I, k * kCycleChunk, std::min(mr, (k + 1) * kCycleChunk));
+        if ((int)I->chunk_done.size() <= k)
+        {
+            cudaEvent_t e;
+            MHD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            I->chunk_done.push_back(e);
+        }
+        MHD_CUDA(cudaEventRecord(I->chunk_done[k], s));
+    }
 }
 
 void host_read(MhdInduction *I, const double *dev, int n)
@@ -741,15 +781,9 @@ int solve_impl(MhdInduction *I, const double *Phi, const double *Ee, const int8_
                        launch_pdl(k_vec_v0, ge, 256, 0, s, ne, I->r.p, sc + 1, I->V.p, I->pd.p, I->mixed ? nullptr : I->zs.p,
                                                    I->mixed ? I->zs32.p : nullptr));
             IND_LAUNCH(I, KI_SCALAR, s,
-                       launch_pdl(k_cycle_init, 1, 1, 0, s, I->ctl.p, std::min(mr, I->p.max_it - total), tol, dtA, I->gv.p, mr + 1, sc + 1));
-            if (!I->prof.on && !I->cycle_tried[I->mode]) build_cycle_graph(I);
-            if (!I->prof.on && I->cycle[I->mode])
-            {
-                MHD_CUDA(cudaGraphLaunch(I->cycle[I->mode], s));
-                I->launches += I->cycle_kernels[I->mode];
-            }
-            else
-                enqueue_cycle(I);
+                       launch_pdl(k_cycle_init, 1, 1, 0, s, I->ctl.p, std::min(mr, I->p.max_it - total), tol, dtA, I->gv.p, mr + 1, sc + 1,
+                                  reinterpret_cast<int *>(I->pinned + 7)));
+            run_cycle(I, std::min(mr, I->p.max_it - total));
             if (mr <= 32) IND_LAUNCH(I, KI_SCALAR, s, launch_pdl(k_backsub_warp, 1, 32, 0, s, I->ctl.p, I->H.p, mr, I->gv.p, I->yv.p, sc + 2));
             else IND_LAUNCH(I, KI_SCALAR, s, k_backsub<<<1, 1, 0, s>>>(I->ctl.p, I->H.p, mr, I->gv.p, I->yv.p, sc + 2));
             if (I->mode == 2)
@@ -792,8 +826,8 @@ void drop_cycle_graphs(MhdInduction *I)
     MHD_CUDA(cudaStreamSynchronize(I->mesh->stream));
     for (int k = 0; k < 3; ++k)
     {
-        if (I->cycle[k]) MHD_CUDA(cudaGraphExecDestroy(I->cycle[k]));
-        I->cycle[k] = nullptr;
+        for (auto &c : I->cycle[k]) MHD_CUDA(cudaGraphExecDestroy(c.exec));
+        I->cycle[k].clear();
         I->cycle_tried[k] = false;
     }
 }

@@ -27,8 +27,12 @@ struct Ctl
 {
     int done, jend, limit, reorth; // reorth: the Gram-Schmidt step of this column needs its second pass
     int n_reorth, pad;             // second passes run in this cycle
+    int *host_done;                // done, for the host (pinned memory)
     double tol, dt;
 };
+// Arnoldi steps that are launched together: with the host one chunk ahead of the device, a cycle that meets the tolerance
+// early leaves at most two chunks of idle launches (about 1.2 us a kernel) instead of the whole restart.
+constexpr int kCycleChunk = 5;
 struct Gate
 {
     const Ctl *ctl = nullptr;
@@ -379,17 +383,24 @@ struct MhdInduction
     double cuct = 0.5;
     mhd::DBuf<double> u_ideal, ide, face3, dte;
     mhd::DBuf<int8_t> imask;
-    // one restart cycle (mr Arnoldi steps) captured as a CUDA graph on the first unprofiled solve of each
-    // kind (mode 0: Jacobi with a scalar dt; 1: Jacobi with the per-edge dt; 2: ILU(0))
+    // the restart cycle's Arnoldi steps in chunks of kCycleChunk, each captured as a CUDA graph on the first unprofiled
+    // solve of each kind (mode 0: Jacobi with a scalar dt; 1: Jacobi with the per-edge dt; 2: ILU(0)); an event per chunk
     int mode = 0;
-    cudaGraphExec_t cycle[3] = {nullptr, nullptr, nullptr};
+    struct Chunk
+    {
+        cudaGraphExec_t exec = nullptr;
+        int64_t kernels = 0;
+    };
+    std::vector<Chunk> cycle[3];
     bool cycle_tried[3] = {false, false, false};
-    int64_t cycle_kernels[3] = {0, 0, 0};
+    std::vector<cudaEvent_t> chunk_done;
     bool capturing = false;
     ~MhdInduction()
     {
-        for (auto &g : cycle)
-            if (g) cudaGraphExecDestroy(g);
+        for (auto &v : cycle)
+            for (auto &c : v)
+                if (c.exec) cudaGraphExecDestroy(c.exec);
+        for (cudaEvent_t e : chunk_done) cudaEventDestroy(e);
         if (pinned) cudaFreeHost(pinned);
     }
 };
