@@ -104,12 +104,8 @@ __device__ __forceinline__ V3 electron_pressure_gradient(const MeshView &m, int3
     {
         const int32_t f = m.c2f_idx[k];
         double pf = pc;
-        const int32_t b = m.f2c_ptr[f];
-        if (m.f2c_ptr[f + 1] - b == 2)
-        {
-            const int32_t o = m.f2c_idx[b] == c ? m.f2c_idx[b + 1] : m.f2c_idx[b];
-            if (m.material[o] == 0) pf = 0.5 * (pf + pe(o));
-        }
+        const int32_t o = m.face_L[f] == c ? m.face_R[f] : m.face_L[f];
+        if (o >= 0 && m.material[o] == 0) pf = 0.5 * (pf + pe(o));
         sum = sum + (pf * static_cast<double>(m.c2f_sgn[k])) * ld3(m.face_area, f);
     }
     const double iv = 1.0 / m.cell_volume[c];

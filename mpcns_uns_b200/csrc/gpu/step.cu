@@ -238,20 +238,31 @@ __global__ void __launch_bounds__(128) k_update(MeshView m, FluidParams p, int s
     }
 }
 
-// mhd::faraday_update on the active faces (Faraday.cpp:15-24); stage 2 averages with Phi0 in place (Solver.cpp:507-508)
+// mhd::faraday_update on the active faces (Faraday.cpp:15-24); stage 2 averages with Phi0 in place (Solver.cpp:507-508).
+// TRI: every face a triangle (f2e row of face f at 3f), the three edge values loaded together; a face is active where one
+// of its two cells is owned.  3.7M faces: 52 -> 28 us, 75% of the copy bandwidth.
+template <bool TRI>
 __global__ void __launch_bounds__(256) k_ct(MeshView m, const double *__restrict__ E, const double *__restrict__ phis,
                                              double *__restrict__ phio, const double *__restrict__ dtp, int stage2)
 {
     pdl_begin();
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nf) return;
-    bool active = false;
-    for (int32_t k = m.f2c_ptr[f]; k < m.f2c_ptr[f + 1]; ++k) active |= m.f2c_idx[k] < m.no_cells;
+    const bool active = m.no_cells == m.nc || (uint32_t)m.face_L[f] < (uint32_t)m.no_cells || (uint32_t)m.face_R[f] < (uint32_t)m.no_cells;
     double v = phis[f];
     if (active)
     {
         double circ = 0.0;
-        for (int32_t k = m.f2e_ptr[f]; k < m.f2e_ptr[f + 1]; ++k) circ += m.f2e_sgn[k] * E[m.f2e_idx[k]];
+        if constexpr (TRI)
+        {
+            const int64_t k = 3 * (int64_t)f;
+            const double e0 = E[m.f2e_idx[k]], e1 = E[m.f2e_idx[k + 1]], e2 = E[m.f2e_idx[k + 2]];
+            circ += m.f2e_sgn[k] * e0;
+            circ += m.f2e_sgn[k + 1] * e1;
+            circ += m.f2e_sgn[k + 2] * e2;
+        }
+        else
+            for (int32_t k = m.f2e_ptr[f]; k < m.f2e_ptr[f + 1]; ++k) circ += m.f2e_sgn[k] * E[m.f2e_idx[k]];
         v -= *dtp * circ;
     }
     phio[f] = stage2 ? 0.5 * (phio[f] + v) : v;
@@ -428,7 +439,7 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
     if (ct && m.nf)
     {
         P.begin(KP_CT, s);
-        launch_pdl(k_ct, grid_for(m.nf, 256), 256, 0, s, m, st->E.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
+        launch_pdl(m.tri_faces ? k_ct<true> : k_ct<false>, grid_for(m.nf, 256), 256, 0, s, m, st->E.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
         MHD_LAUNCH_CHECK();
         P.end(KP_CT, s);
         ++st->launches;
@@ -861,7 +872,7 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
         if (m.nf)
         {
             st->prof.begin(KP_CT, s);
-            launch_pdl(k_ct, grid_for(m.nf, 256), 256, 0, s, m, st->E_impl.p, st->phi0.p, st->phi0.p, st->scal.p, 0);
+            launch_pdl(m.tri_faces ? k_ct<true> : k_ct<false>, grid_for(m.nf, 256), 256, 0, s, m, st->E_impl.p, st->phi0.p, st->phi0.p, st->scal.p, 0);
             MHD_LAUNCH_CHECK();
             st->prof.end(KP_CT, s);
             ++st->launches;
