@@ -333,6 +333,8 @@ struct MhdMesh
     mhd::MeshView v{};
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaStream_t side = nullptr; // a stage's EMF passes (StageFork); joined to stream before a call returns
+    cudaEvent_t ev_prep = nullptr, ev_face = nullptr, ev_ct = nullptr;
     mhd::DBuf<int32_t> c2f_ptr, c2f_idx, f2e_ptr, f2e_idx, e2f_ptr, e2f_idx, f2c_ptr, f2c_idx, face_L, face_R, ec_ptr, ec_cell, st_nb,
         cfa_idx;
     mhd::DBuf<int8_t> c2f_sgn, f2e_sgn, e2f_sgn, f2c_sgn, material, face_kind, edge_mode, edge_uct, st_valid, cfa_sgn;

@@ -226,6 +226,9 @@ MhdMesh::~MhdMesh()
 {
     if (pinned) cudaFreeHost(pinned);
     if (own_stream && stream) cudaStreamDestroy(stream);
+    if (side) cudaStreamDestroy(side);
+    for (cudaEvent_t e : {ev_prep, ev_face, ev_ct})
+        if (e) cudaEventDestroy(e);
 }
 
 using namespace mhd;
@@ -382,6 +385,8 @@ int mhd_gpu_mesh_create(const MhdMeshDesc *d, MhdMesh **out)
         }
         MHD_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
         m->own_stream = true;
+        MHD_CUDA(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
+        for (cudaEvent_t *e : {&m->ev_prep, &m->ev_face, &m->ev_ct}) MHD_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         MHD_CUDA(cudaMallocHost(&m->pinned, 64 * sizeof(double)));
         // stencil tables
         m->st_nb.alloc(c2fp[nc]);

@@ -1190,13 +1190,41 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
     }
     float4 *W4 = reinterpret_cast<float4 *>(st->W32.p);
     if (!prepared) mixed_prepare(st, Us, phis, cfl, dt_max, false);
-    // face EMF candidates first: with the J x B force on, this pass also leaves the face terms of the
-    // cell current that the update gathers
-    P.begin(KP_FACE_CAND, s);
-    launch_pdl(k_mx_face_cand, gf, 128, 0, s, m, st->up32.p, st->bt32.p, st->bi32.p, phis, st->phi_add.p, st->Ef32.p,
-                                      st->src.on ? st->g32.p : nullptr, W4, st->src.ambi ? st->d32.p : nullptr);
-    MHD_LAUNCH_CHECK();
-    P.end(KP_FACE_CAND, s);
+    StageFork fork(st, true);
+    cudaStream_t se = fork.emf;
+    // the EMF chain in two halves, enqueued between the fluid's passes so that neither chain waits for the host.  With the
+    // J x B force on, the face candidates' pass also leaves the face terms of the cell current that the update gathers
+    auto emf_faces = [&] {
+        P.begin(KP_FACE_CAND, se);
+        launch_pdl(k_mx_face_cand, gf, 128, 0, se, m, st->up32.p, st->bt32.p, st->bi32.p, phis, st->phi_add.p, st->Ef32.p,
+                   st->src.on ? st->g32.p : nullptr, W4, st->src.ambi ? st->d32.p : nullptr);
+        MHD_LAUNCH_CHECK();
+        P.end(KP_FACE_CAND, se);
+        fork.faces_done();
+    };
+    auto emf_edges = [&] {
+        const float3 Einf = make_float3(static_cast<float>(-(st->prm.u_inf[1] * st->prm.B_imf[2] - st->prm.u_inf[2] * st->prm.B_imf[1])),
+                                        static_cast<float>(-(st->prm.u_inf[2] * st->prm.B_imf[0] - st->prm.u_inf[0] * st->prm.B_imf[2])),
+                                        static_cast<float>(-(st->prm.u_inf[0] * st->prm.B_imf[1] - st->prm.u_inf[1] * st->prm.B_imf[0])));
+        P.begin(KP_EDGE_EMF, se);
+        launch_pdl(k_mx_edge, ge, 128, 0, se, m, st->Ef32.p, st->up32.p, static_cast<float>(st->prm.cuct), Einf, st->E32.p);
+        MHD_LAUNCH_CHECK();
+        if (st->src.ambi)
+        {
+            if (mv.nn)
+                launch_pdl(k_mx_node_pressure, grid_for(mv.nn, 128), 128, 0, se, mv.nn, mv.n2c_ptr, mv.n2c_cell, mv.cell_volume, W4, st->pn.p,
+                                                                        st->pok.p);
+            launch_pdl(k_mx_ambipolar, grid_for(m.ne, 128), 128, 0, se, m, p, W4, mv.ec_weight, mv.e_nodes, st->pn.p, st->pok.p,
+                                                                static_cast<float>(st->prm.pressure_coef), st->E32.p);
+            MHD_LAUNCH_CHECK();
+            st->launches += 1 + (mv.nn ? 1 : 0);
+        }
+        P.end(KP_EDGE_EMF, se);
+        P.begin(KP_CT, se);
+        launch_pdl(k_mx_ct, grid_for(m.nf, 256), 256, 0, se, m.nf, st->mt.fe.p, st->E32.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
+        MHD_LAUNCH_CHECK();
+        P.end(KP_CT, se);
+    };
     for (int s0 = 0; s0 < st->nsp; s0 += st->group)
     {
         const int ng = std::min(st->group, st->nsp - s0);
@@ -1205,10 +1233,16 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
                                                                                    reinterpret_cast<float4 *>(st->grad32.p));
         MHD_LAUNCH_CHECK();
         P.end(KP_GRAD, s);
+        if (s0 == 0) emf_faces();
         P.begin(KP_FLUX, s);
         launch_pdl(k_mx_flux, grid_for(static_cast<int64_t>(m.nf) * ng, 128), 128, 0, s, m, p, s0, ng, st->grad32.p, st->F32.p);
         MHD_LAUNCH_CHECK();
         P.end(KP_FLUX, s);
+        if (s0 == 0)
+        {
+            emf_edges();
+            fork.before_update();
+        }
         P.begin(KP_UPDATE, s);
         // the instance with the closing gyration fused carries its registers; the other stages use the lean one
         auto upd = gyrate_close && s0 == 0 ? k_mx_update<true> : k_mx_update<false>;
@@ -1219,27 +1253,7 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
         P.end(KP_UPDATE, s);
         st->launches += 3;
     }
-    const float3 Einf = make_float3(static_cast<float>(-(st->prm.u_inf[1] * st->prm.B_imf[2] - st->prm.u_inf[2] * st->prm.B_imf[1])),
-                                    static_cast<float>(-(st->prm.u_inf[2] * st->prm.B_imf[0] - st->prm.u_inf[0] * st->prm.B_imf[2])),
-                                    static_cast<float>(-(st->prm.u_inf[0] * st->prm.B_imf[1] - st->prm.u_inf[1] * st->prm.B_imf[0])));
-    P.begin(KP_EDGE_EMF, s);
-    launch_pdl(k_mx_edge, ge, 128, 0, s, m, st->Ef32.p, st->up32.p, static_cast<float>(st->prm.cuct), Einf, st->E32.p);
-    MHD_LAUNCH_CHECK();
-    if (st->src.ambi)
-    {
-        if (mv.nn)
-            launch_pdl(k_mx_node_pressure, grid_for(mv.nn, 128), 128, 0, s, mv.nn, mv.n2c_ptr, mv.n2c_cell, mv.cell_volume, W4, st->pn.p,
-                                                                    st->pok.p);
-        launch_pdl(k_mx_ambipolar, grid_for(m.ne, 128), 128, 0, s, m, p, W4, mv.ec_weight, mv.e_nodes, st->pn.p, st->pok.p,
-                                                            static_cast<float>(st->prm.pressure_coef), st->E32.p);
-        MHD_LAUNCH_CHECK();
-        st->launches += 1 + (mv.nn ? 1 : 0);
-    }
-    P.end(KP_EDGE_EMF, s);
-    P.begin(KP_CT, s);
-    launch_pdl(k_mx_ct, grid_for(m.nf, 256), 256, 0, s, m.nf, st->mt.fe.p, st->E32.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
-    MHD_LAUNCH_CHECK();
-    P.end(KP_CT, s);
+    fork.join();
     st->launches += 3;
 }
 } // namespace mhd

@@ -142,6 +142,45 @@ __device__ __forceinline__ void cfl_reduce(const CflOut &o, double v, bool bad)
 }
 #endif
 
+// A stage's two chains after the prepare pass: the fluid's (face values, fluxes, update) on the mesh's stream and the EMF's
+// (cell current, face candidates, edge EMF, CT) on the mesh's side stream.  They share their inputs and meet twice: the
+// update reads what the EMF chain's first passes leave, and the stage ends when both have.  A pass of a small mesh is a few
+// waves of blocks whose last one leaves most SMs idle, and its launch costs as much as its work: there the other chain's
+// blocks fill the gaps.  A pass that saturates DRAM gains nothing and loses nothing.  Per step, one stream -> two:
+// mixed 24k cells 46 -> 41 us, 221k 251 -> 205 us, 14.2M 10.94 -> 10.96 ms; FP64 24k 81 -> 75 us, 1.8M 3.25 -> 3.22 ms.
+// So every size takes two streams, except while the passes are timed one by one by the profiler.
+struct StageFork
+{
+    MhdMesh *m;
+    cudaStream_t main, emf;
+    bool on;
+    StageFork(MhdState *s, bool fork) : m(s->mesh), main(s->mesh->stream), emf(s->mesh->stream), on(fork && !s->prof.on)
+    {
+        if (!on) return;
+        emf = m->side;
+        MHD_CUDA(cudaEventRecord(m->ev_prep, main));
+        MHD_CUDA(cudaStreamWaitEvent(emf, m->ev_prep, 0));
+    }
+    void faces_done() // what the update reads has been enqueued on emf
+    {
+        if (on) MHD_CUDA(cudaEventRecord(m->ev_face, emf));
+    }
+    void before_update()
+    {
+        if (on) MHD_CUDA(cudaStreamWaitEvent(main, m->ev_face, 0));
+    }
+    void join()
+    {
+        if (!on) return;
+        MHD_CUDA(cudaEventRecord(m->ev_ct, emf));
+        MHD_CUDA(cudaStreamWaitEvent(main, m->ev_ct, 0));
+        on = false;
+    }
+    ~StageFork() // an exception between: the side stream still rejoins
+    {
+        if (on && cudaEventRecord(m->ev_ct, emf) == cudaSuccess) cudaStreamWaitEvent(main, m->ev_ct, 0);
+    }
+};
 void mixed_setup(MhdState *st);
 // one FP64 stage (Us, phis) -> (Uo, phio) at the step size in st->scal[0]; stage2 averages with Uo, phio in place
 void fp64_stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2);

@@ -342,11 +342,6 @@ void prepare_cfl(MhdState *st, const double *Us, const double *phis, bool cfl, d
         // grad p_e and the nodal p_e below need the primitives before the gyration
         launch_prepare(st, Us, phis, cfl, dt_max, turned && !st->src.ambi);
         ++st->launches;
-        if (st->src.on) // J of the induced field (Solver.cpp:123)
-        {
-            launch_cell_current(m, st->bind.p, st->J.p, s);
-            ++st->launches;
-        }
         if (st->src.ambi && !st->mixed) // grad p_e (Solver.cpp:124) and the nodal p_e of the ambipolar EMF
         {
             launch_dpe(m, st->W.p, st->dpe.p, s);
@@ -375,6 +370,48 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
                      st->src.ambi ? st->dpe.p : nullptr,
                      st->src.chem && st->photo.n ? st->photo.p : nullptr,
                      st->src.chem && st->vst.n ? st->vst.p : nullptr};
+    StageFork fork(st, m.nc > 0);
+    cudaStream_t se = fork.emf;
+    // the EMF chain in two halves, enqueued between the fluid's passes so that neither chain waits for the host
+    auto emf_faces = [&] {
+        if (st->src.on && m.nc) // J of the induced field (Solver.cpp:123)
+        {
+            P.begin(KP_PREPARE, se);
+            launch_cell_current(m, st->bind.p, st->J.p, se);
+            P.end(KP_PREPARE, se);
+            ++st->launches;
+        }
+        fork.faces_done();
+        P.begin(KP_FACE_CAND, se);
+        launch_face_candidate(m, st->up.p, st->btot.p, st->bind.p, phis, st->phi_add.p, st->Ef.p, se, st->efgeo.n ? st->pa.p : nullptr,
+                              st->sw_face);
+        P.end(KP_FACE_CAND, se);
+        st->launches += m.nf ? 1 : 0;
+    };
+    auto emf_edges = [&] {
+        const V3 ui = mk(st->prm.u_inf[0], st->prm.u_inf[1], st->prm.u_inf[2]), bi = mk(st->prm.B_imf[0], st->prm.B_imf[1], st->prm.B_imf[2]);
+        const V3 Einf = -1.0 * cross(ui, bi);
+        P.begin(KP_EDGE_EMF, se);
+        AmbArgs amb;
+        amb.on = st->src.ambi;
+        amb.p = st->src;
+        amb.W = st->W.p;
+        amb.pn = st->pn.p;
+        amb.pok = st->pok.p;
+        launch_edge_emf_assign(m, st->Ef.p, st->up.p, phis, st->prm.cuct, Einf, st->E.p, se, st->mres.n ? st->mres.p : nullptr, amb,
+                               st->sw_edge, st->efgeo.n ? st->efgeo.p : nullptr, st->efgeo.n ? st->pa.p : nullptr);
+        P.end(KP_EDGE_EMF, se);
+        st->launches += m.ne ? 1 : 0;
+        if (ct && m.nf)
+        {
+            P.begin(KP_CT, se);
+            launch_pdl(m.tri_faces ? k_ct<true> : k_ct<false>, grid_for(m.nf, 256), 256, 0, se, m, st->E.p, phis, phio, st->scal.p,
+                       stage2 ? 1 : 0);
+            MHD_LAUNCH_CHECK();
+            P.end(KP_CT, se);
+            ++st->launches;
+        }
+    };
     for (int s0 = 0; s0 < nsp; s0 += st->group)
     {
         const int ng = std::min(st->group, nsp - s0);
@@ -404,10 +441,16 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
             if (log && st->fv.n && st->floor_flags) launch_face_values(m, gp, Wg, false, nullptr, st->fv.p, s);
         }
         P.end(KP_GRAD, s);
+        if (s0 == 0) emf_faces();
         P.begin(KP_FLUX, s);
         if (faces) launch_face_flux_fv(m, gp, st->fv.p, st->F.p, s);
         else launch_face_flux(m, gp, Wg, SField<const double>{st->grad.p, 15 * nc, 1, nc}, st->F.p, s);
         P.end(KP_FLUX, s);
+        if (s0 == 0)
+        {
+            emf_edges();
+            fork.before_update();
+        }
         if (m.nc)
         {
             P.begin(KP_UPDATE, s);
@@ -419,31 +462,7 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
         }
         st->launches += (st->prm.second_order && m.nc ? 1 : 0) + (m.nf ? 1 : 0) + (m.nc ? 1 : 0);
     }
-    const V3 ui = mk(st->prm.u_inf[0], st->prm.u_inf[1], st->prm.u_inf[2]), bi = mk(st->prm.B_imf[0], st->prm.B_imf[1], st->prm.B_imf[2]);
-    const V3 Einf = -1.0 * cross(ui, bi);
-    P.begin(KP_FACE_CAND, s);
-    launch_face_candidate(m, st->up.p, st->btot.p, st->bind.p, phis, st->phi_add.p, st->Ef.p, s, st->efgeo.n ? st->pa.p : nullptr,
-                          st->sw_face);
-    P.end(KP_FACE_CAND, s);
-    P.begin(KP_EDGE_EMF, s);
-    AmbArgs amb;
-    amb.on = st->src.ambi;
-    amb.p = st->src;
-    amb.W = st->W.p;
-    amb.pn = st->pn.p;
-    amb.pok = st->pok.p;
-    launch_edge_emf_assign(m, st->Ef.p, st->up.p, phis, st->prm.cuct, Einf, st->E.p, s, st->mres.n ? st->mres.p : nullptr, amb,
-                           st->sw_edge, st->efgeo.n ? st->efgeo.p : nullptr, st->efgeo.n ? st->pa.p : nullptr);
-    P.end(KP_EDGE_EMF, s);
-    st->launches += (m.nf ? 1 : 0) + (m.ne ? 1 : 0);
-    if (ct && m.nf)
-    {
-        P.begin(KP_CT, s);
-        launch_pdl(m.tri_faces ? k_ct<true> : k_ct<false>, grid_for(m.nf, 256), 256, 0, s, m, st->E.p, phis, phio, st->scal.p, stage2 ? 1 : 0);
-        MHD_LAUNCH_CHECK();
-        P.end(KP_CT, s);
-        ++st->launches;
-    }
+    fork.join();
 }
 
 } // namespace
