@@ -274,9 +274,10 @@ __device__ __forceinline__ void rusanov32(const F5 &L, const F5 &R, float3 n, fl
 
 // per-cell primitives (FP32, 32 bytes per species) and the charge-weighted velocity u+ of cell c.  NSP: the number of
 // species, whose primitives then stay in w (0: any number, re-read where they are needed); store: write W and up.
-template <int NSP>
-__device__ __forceinline__ void mx_prims(const MxParams &p, int64_t n, const double *__restrict__ U, float4 *__restrict__ W,
-                                         float4 *__restrict__ up, int32_t c, bool fluid, F5 (&w5)[NSP ? NSP : 1], bool store = true)
+// U(s, q): the cell's conservative value q of species s.
+template <int NSP, class Cons>
+__device__ __forceinline__ void mx_prims(const MxParams &p, int64_t n, const Cons &U, float4 *__restrict__ W, float4 *__restrict__ up,
+                                         int32_t c, bool fluid, F5 (&w5)[NSP ? NSP : 1], bool store = true)
 {
     const int nsp = NSP ? NSP : p.nsp;
     float ne = 0.f;
@@ -284,11 +285,10 @@ __device__ __forceinline__ void mx_prims(const MxParams &p, int64_t n, const dou
 #pragma unroll
     for (int s = 0; s < nsp; ++s)
     {
-        const double *Us = U + (int64_t)s * 5 * n;
-        const double r = fmax(Us[c], p.rho_floor_d);
+        const double r = fmax(U(s, 0), p.rho_floor_d);
         const double ir = 1.0 / r;
-        const double u = Us[n + c] * ir, v = Us[2 * n + c] * ir, w = Us[3 * n + c] * ir;
-        const double pr = fmax((p.gamma_d - 1.0) * (Us[4 * n + c] - 0.5 * r * (u * u + v * v + w * w)), p.p_floor_d);
+        const double u = U(s, 1) * ir, v = U(s, 2) * ir, w = U(s, 3) * ir;
+        const double pr = fmax((p.gamma_d - 1.0) * (U(s, 4) - 0.5 * r * (u * u + v * v + w * w)), p.p_floor_d);
         const F5 q{static_cast<float>(r), static_cast<float>(u), static_cast<float>(v), static_cast<float>(w), static_cast<float>(pr)};
         if (NSP) w5[s] = q;
         if (!NSP || store)
@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(128) k_mx_prepare(MV m, MxParams p, const doub
     {
         F5 w5[NSP ? NSP : 1];
         const int mat = m.material[c];
-        mx_prims<NSP>(p, n, U, W, up, c, mat == 0, w5, !CFL || !cfl.turned || c >= m.no_cells || mat == 1);
+        auto cons = [&](int s, int q) { return U[((int64_t)s * 5 + q) * n + c]; };
+        mx_prims<NSP>(p, n, cons, W, up, c, mat == 0, w5, !CFL || !cfl.turned || c >= m.no_cells || mat == 1);
         const int4 fi = *reinterpret_cast<const int4 *>(m.c2f_idx + 4 * (int64_t)c);
         const float ph[4] = {static_cast<float>(phi[fi.x]), static_cast<float>(phi[fi.y]), static_cast<float>(phi[fi.z]),
                              static_cast<float>(phi[fi.w])};
@@ -401,9 +402,10 @@ __global__ void __launch_bounds__(128) k_mx_prepare(MV m, MxParams p, const doub
 }
 
 // The opening half-step gyration (mercury::gyrate, FP64 on the FP64 state, FP32 total field) with the
-// primitives and u+ of the cells it turns renewed, so that stage 1 starts prepared (B_ind and B_tot
-// depend on Phi alone)
-__global__ void __launch_bounds__(128) k_mx_gyrate(MV m, MxParams p, SrcParams sp, const float4 *__restrict__ bt,
+// primitives and u+ of the cells it turns renewed from the values at hand, so that stage 1 starts prepared (B_ind and
+// B_tot depend on Phi alone).  At the DRAM rate with 28 warps an SM: 14.2M cells 695 us with 20 warps and U read twice,
+// 554 us now (64 registers: 600 us)
+__global__ void __launch_bounds__(128, 7) k_mx_gyrate(MV m, MxParams p, SrcParams sp, const float4 *__restrict__ bt,
                                                    const double *__restrict__ dtp, double scale, double *__restrict__ U,
                                                    float4 *__restrict__ W, float4 *__restrict__ up)
 {
@@ -424,7 +426,8 @@ __global__ void __launch_bounds__(128) k_mx_gyrate(MV m, MxParams p, SrcParams s
         U[(5 + q) * n + c] = un[q];
     }
     F5 w5[2];
-    mx_prims<2>(p, n, U, W, up, c, m.material[c] == 0, w5);
+    auto cons = [&](int s, int q) { return s ? un[q] : uh[q]; };
+    mx_prims<2>(p, n, cons, W, up, c, m.material[c] == 0, w5);
 }
 
 // limited face values (see below) of cell c for species s0 + g of a group of ng: FV[(q*n + c)*ng + g] holds
@@ -914,7 +917,7 @@ __global__ void __launch_bounds__(128) k_mx_flux(MV m, MxParams p, int s0, int n
 // state, with the total field of the stage-2 prepare) applied to the cell's two ions before they are
 // written, instead of in a pass of its own
 template <bool GYR>
-__global__ void __launch_bounds__(128) k_mx_update(MV m, MxParams p, int s0, int ng, const float *__restrict__ F,
+__global__ void __launch_bounds__(128, 5) k_mx_update(MV m, MxParams p, int s0, int ng, const float *__restrict__ F,
                                                    const double *__restrict__ Ub, double *__restrict__ Uo, const double *__restrict__ dtp,
                                                    int stage2, const float4 *__restrict__ G,
                                                    const float4 *__restrict__ bt, SrcParams sp, int gyr, const float4 *__restrict__ D,

@@ -188,9 +188,9 @@ __device__ __forceinline__ void gyrate_cell(const SrcParams &p, V3 b, double dt,
 // Per-cell part of Solver::prepare (Solver.cpp:101-118): primitives of every species and the
 // charge-weighted ion velocity u+ (mhd::Scales::numinfo generalised to n species).  NSP: the number of species, whose
 // primitives then stay in w (and go to W if store); 0: any number, the number densities recomputed from the primitives
-// just written.
-template <int NSP>
-__device__ __forceinline__ void prepare_prims(const FluidParams &p, const double *__restrict__ mass, double M_ref, SField<const double> U,
+// just written.  U(s, c, q): the conservative values.
+template <int NSP, class Cons>
+__device__ __forceinline__ void prepare_prims(const FluidParams &p, const double *__restrict__ mass, double M_ref, const Cons &U,
                                               SField<double> W, int32_t c, bool fluid, double *u, Prim5 (&w)[NSP ? NSP : 1], bool store = true)
 {
     double ne = 0;
@@ -229,7 +229,6 @@ struct Reprepare
     FluidParams fp;
     const double *mass = nullptr;
     double M_ref = 1;
-    SField<const double> U;
     SField<double> W;
     double *up = nullptr;
 };

@@ -354,7 +354,7 @@ void prepare_cfl(MhdState *st, const double *Us, const double *phis, bool cfl, d
 }
 
 void stage(MhdState *st, const double *Us, const double *phis, double *Uo, double *phio, bool stage2, bool cfl, double dt_max,
-           bool prepared = false, bool ct = true)
+           bool prepared = false, bool ct = true, bool gyrate_close = false)
 {
     MhdMesh *mesh = st->mesh;
     const MeshView &m = mesh->v;
@@ -461,6 +461,13 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
             P.end(KP_UPDATE, s);
         }
         st->launches += (st->prm.second_order && m.nc ? 1 : 0) + (m.nf ? 1 : 0) + (m.nc ? 1 : 0);
+    }
+    if (gyrate_close) // the closing half-step gyration of Uo with this stage's Btot, beside the end of the EMF chain
+    {
+        P.begin(KP_GYRATE, s);
+        launch_gyrate(m, st->src, st->btot.p, nullptr, st->scal.p, 0.5, Uo, s);
+        P.end(KP_GYRATE, s);
+        st->launches += m.no_cells ? 1 : 0;
     }
     fork.join();
 }
@@ -796,7 +803,6 @@ int mhd_gpu_step_rk2(MhdState *st, double dt_fixed, double dt_max, double *dt_us
                 rp.fp = st->fp;
                 rp.mass = st->mass.p;
                 rp.M_ref = st->prm.M_ref;
-                rp.U = soa_cstate(st->U0.p, m.nc);
                 rp.W = soa_state(st->W.p, m.nc);
                 rp.up = st->up.p;
                 st->prof.begin(KP_GYRATE, s);
@@ -805,15 +811,8 @@ int mhd_gpu_step_rk2(MhdState *st, double dt_fixed, double dt_max, double *dt_us
                 st->launches += m.no_cells ? 1 : 0;
             }
             stage(st, st->U0.p, st->phi0.p, st->U1.p, st->phi1.p, false, cfl && !split, dt_max, split);
-            stage(st, st->U1.p, st->phi1.p, st->U0.p, st->phi0.p, true, false, dt_max);
-            if (split)
-            {
-                st->prof.begin(KP_GYRATE, s);
-                launch_gyrate(m, st->src, st->btot.p, nullptr, st->scal.p, 0.5, st->U0.p, s);
-                st->prof.end(KP_GYRATE, s);
-            }
+            stage(st, st->U1.p, st->phi1.p, st->U0.p, st->phi0.p, true, false, dt_max, false, true, split);
         }
-        if (split && m.no_cells && !st->mixed) ++st->launches; // the FP64 closing gyration
         if (dt_used) read_dt(st, dt_used);
     });
 }
@@ -849,7 +848,6 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
             rp.fp = st->fp;
             rp.mass = st->mass.p;
             rp.M_ref = st->prm.M_ref;
-            rp.U = soa_cstate(st->U0.p, m.nc);
             rp.W = soa_state(st->W.p, m.nc);
             rp.up = st->up.p;
             st->prof.begin(KP_GYRATE, s);
@@ -859,7 +857,7 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
         }
         // rhs and forward Euler of the fluid with floors, in place; E = the explicit EMF (ideal, ambipolar,
         // boundary values); no CT yet
-        stage(st, st->U0.p, st->phi0.p, st->U0.p, st->phi0.p, false, cfl && !split, dt_max, split, false);
+        stage(st, st->U0.p, st->phi0.p, st->U0.p, st->phi0.p, false, cfl && !split, dt_max, split, false, split);
         // the implicit linear terms with the total EMF as the unknown (:250-266)
         st->ne_eff.alloc(std::max<size_t>(1, (size_t)m.nc));
         st->E_impl.alloc(std::max<size_t>(1, (size_t)m.ne));
@@ -886,8 +884,8 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
         if (rcs == MHD_ENOCONV) status = MHD_ENOCONV;
         if (iterations) *iterations = it;
         if (rel_res) *rel_res = rr;
-        // faraday_update with the implicit EMF (:269), then the closing half-step gyration with the Btot of
-        // the step's prepare (:274)
+        // faraday_update with the implicit EMF (:269); the closing half-step gyration with the Btot of the step's prepare
+        // (:274) reads neither and is done beside the explicit EMF
         if (m.nf)
         {
             st->prof.begin(KP_CT, s);
@@ -895,13 +893,6 @@ int mhd_gpu_step_semi_implicit(MhdState *st, MhdInduction *ind, double dt_fixed,
             MHD_LAUNCH_CHECK();
             st->prof.end(KP_CT, s);
             ++st->launches;
-        }
-        if (split)
-        {
-            st->prof.begin(KP_GYRATE, s);
-            launch_gyrate(m, st->src, st->btot.p, nullptr, st->scal.p, 0.5, st->U0.p, s);
-            st->prof.end(KP_GYRATE, s);
-            st->launches += m.no_cells ? 1 : 0;
         }
         if (dt_used) *dt_used = dt;
         MHD_CUDA(cudaStreamSynchronize(s));
