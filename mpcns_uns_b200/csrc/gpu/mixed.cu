@@ -31,10 +31,10 @@ struct MV
     const int32_t *c2f_idx, *cfa_idx, *t_nb, *face_L, *face_R, *f2c_ptr, *f2c_idx, *f2e_ptr, *f2e_idx, *e2f_ptr, *e2f_idx, *ec_ptr,
         *ec_cell;
     const int8_t *c2f_sgn, *cfa_sgn, *t_sg, *material, *face_kind, *edge_mode, *st_valid, *f2c_sgn, *f2e_sgn, *emode;
-    const float *K, *recon, *fdx, *vol_inv;
+    const float *K, *recon, *vol_inv;
     const float4 *fn, *eth, *emn;
     const float2 *esw;
-    const char2 *fslot;
+    const int4 *frec; // the faces' records: entries 4 c + j of their cells, boundary kind
     const double *cell_volume; // FP64: the update divides the FP64-summed fluxes by it
 };
 
@@ -47,9 +47,9 @@ MV make_view(const MeshView &m, const MixedTables &t)
     v.e2f_idx = m.e2f_idx; v.ec_ptr = m.ec_ptr; v.ec_cell = m.ec_cell;
     v.c2f_sgn = m.c2f_sgn; v.cfa_sgn = m.cfa_sgn; v.t_sg = m.t_sg; v.material = m.material; v.face_kind = m.face_kind;
     v.edge_mode = m.edge_mode; v.st_valid = m.st_valid; v.f2c_sgn = m.f2c_sgn; v.f2e_sgn = m.f2e_sgn;
-    v.K = t.K.p; v.recon = t.recon.p; v.fdx = t.fdx.p; v.vol_inv = t.vol_inv.p;
+    v.K = t.K.p; v.recon = t.recon.p; v.vol_inv = t.vol_inv.p;
     v.fn = t.fn.p; v.eth = t.eth.p; v.emn = t.emn.p; v.esw = t.esw.p; v.emode = t.emode.p;
-    v.fslot = t.fslot.p;
+    v.frec = m.frec;
     v.cell_volume = m.cell_volume;
     return v;
 }
@@ -125,31 +125,13 @@ __global__ void k_mx_cells(MeshView m, float *K, float *recon, float *vol_inv)
             recon[(3 * j + a) * n + c] = A[j] > 0 ? static_cast<float>(I[a][0] * nn[j].x + I[a][1] * nn[j].y + I[a][2] * nn[j].z) : 0.f;
 }
 
-__global__ void k_mx_faces(MeshView m, float4 *fn, float *fdx, char2 *fslot)
+__global__ void k_mx_faces(MeshView m, float4 *fn)
 {
     const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= m.nf) return;
-    // position of f in the c2f rows of its L and R cells (the face-value slot of k_mx_grad)
-    {
-        const int32_t L = m.face_L[f], R = m.face_R[f];
-        signed char jl = 0, jr = 0;
-        for (int j = 0; j < 4; ++j)
-        {
-            if (L >= 0 && m.c2f_idx[4 * (int64_t)L + j] == f) jl = static_cast<signed char>(j);
-            if (R >= 0 && m.c2f_idx[4 * (int64_t)R + j] == f) jr = static_cast<signed char>(j);
-        }
-        fslot[f] = make_char2(jl, jr);
-    }
-    const int64_t n = m.nf;
     const double A = m.face_area_mag[f];
     const V3 nr = (1.0 / A) * ld3(m.face_area, f);
     fn[f] = make_float4(static_cast<float>(nr.x), static_cast<float>(nr.y), static_cast<float>(nr.z), static_cast<float>(A));
-    const V3 xf = ld3(m.face_center, f);
-    const int32_t L = m.face_L[f], R = m.face_R[f];
-    const V3 dL = L >= 0 ? xf - ld3(m.cell_center, L) : mk(0, 0, 0);
-    const V3 dR = R >= 0 ? xf - ld3(m.cell_center, R) : mk(0, 0, 0);
-    fdx[0 * n + f] = static_cast<float>(dL.x); fdx[1 * n + f] = static_cast<float>(dL.y); fdx[2 * n + f] = static_cast<float>(dL.z);
-    fdx[3 * n + f] = static_cast<float>(dR.x); fdx[4 * n + f] = static_cast<float>(dR.y); fdx[5 * n + f] = static_cast<float>(dR.z);
 }
 
 // Orthonormal basis (e1, e2) of the plane normal to the unit tangent th, built in single precision; the
@@ -430,10 +412,17 @@ __global__ void __launch_bounds__(128, 7) k_mx_gyrate(MV m, MxParams p, SrcParam
     mx_prims<2>(p, n, cons, W, up, c, m.material[c] == 0, w5);
 }
 
-// limited face values (see below) of cell c for species s0 + g of a group of ng: FV[(q*n + c)*ng + g] holds
+// limited face values (see below) of cell c for species s0 + g of a group of NG: FV[(q*n + c)*NG + g] holds
 // variable q at the cell's four faces (c2f order) as one float4
-__device__ __forceinline__ void mx_grad_one(const MV &m, const MxParams &p, int s0, int g, int ng, int32_t c,
-                                            const float4 *__restrict__ W, float4 *__restrict__ FV)
+template <int NG>
+__device__ __forceinline__ void mx_store_fv(float4 *__restrict__ FV, int64_t n, int32_t c, int g, const float (&fv)[5][4])
+{
+#pragma unroll
+    for (int q = 0; q < 5; ++q) FV[(q * n + c) * NG + g] = make_float4(fv[q][0], fv[q][1], fv[q][2], fv[q][3]);
+}
+template <int NG>
+__device__ __forceinline__ void mx_grad_one(const MV &m, const MxParams &p, int s0, int g, int32_t c, const float4 *__restrict__ W,
+                                            float4 *__restrict__ FV)
 {
     const int s = s0 + g;
     const int64_t n = m.nc;
@@ -443,15 +432,17 @@ __device__ __forceinline__ void mx_grad_one(const MV &m, const MxParams &p, int 
         const float4 a = Ws[2 * (int64_t)cc], b = Ws[2 * (int64_t)cc + 1];
         q5[0] = a.x; q5[1] = a.y; q5[2] = a.z; q5[3] = a.w; q5[4] = b.x;
     };
-    float4 *out = FV + (int64_t)c * ng + g;
-    const int64_t qs = n * ng; // stride of variable q
+    float fv[5][4];
     if (c >= m.no_cells || !m.st_valid[c])
     {
         // zero gradient: every face value is the cell value
         float w5[5];
         prim(c, w5);
 #pragma unroll
-        for (int q = 0; q < 5; ++q) out[q * qs] = make_float4(w5[q], w5[q], w5[q], w5[q]);
+        for (int q = 0; q < 5; ++q)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fv[q][j] = w5[q];
+        mx_store_fv<NG>(FV, n, c, g, fv);
         return;
     }
     int32_t nb[4];
@@ -489,7 +480,6 @@ __device__ __forceinline__ void mx_grad_one(const MV &m, const MxParams &p, int 
     // positivity test) instead of the gradient.  The face that sets the Barth-Jespersen psi is snapped to its
     // bound, which exact arithmetic gives (w + (b - w)/dl * dl = b): near an absorbing wall the bound is the
     // 1e-12 floor state and the single-precision sum w + psi dl, with w ~ 1e-3, could not resolve it.
-    float fv[5][4];
 #pragma unroll
     for (int q = 0; q < 5; ++q)
     {
@@ -549,24 +539,22 @@ __device__ __forceinline__ void mx_grad_one(const MV &m, const MxParams &p, int 
     for (int j = 0; j < 4; ++j) ok[j] = fv[0][j] > 0.f && fv[4][j] > 0.f;
 #pragma unroll
     for (int q = 0; q < 5; ++q)
-        out[q * qs] = make_float4(ok[0] ? fv[q][0] : wc[q], ok[1] ? fv[q][1] : wc[q], ok[2] ? fv[q][2] : wc[q], ok[3] ? fv[q][3] : wc[q]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) fv[q][j] = ok[j] ? fv[q][j] : wc[q];
+    mx_store_fv<NG>(FV, n, c, g, fv);
 }
 
 // Rusanov face flux times |A| of face f for species s0 + g of a group of ng: F[(f*ng + g)*5 + q], so that a
 // face's fluxes of the whole group are one contiguous record for the update's gather
-__device__ __forceinline__ void mx_flux_one(const MV &m, const MxParams &p, int s0, int g, int ng, int32_t f,
+template <int NG>
+__device__ __forceinline__ void mx_flux_one(const MV &m, const MxParams &p, int s0, int g, int32_t f,
                                             const float *__restrict__ FV, float *__restrict__ F)
 {
     const int s = s0 + g;
-    const int64_t n = m.nc;
-    float *Fo = F + ((int64_t)f * ng + g) * 5;
-    const int kind = m.face_kind[f];
-    const int32_t p0 = m.f2c_ptr[f], cnt = m.f2c_ptr[f + 1] - p0;
-    const int32_t L = m.face_L[f], R = m.face_R[f];
-    bool any = false;
-    if (L >= 0) any |= L < m.no_cells && m.material[L] == 0;
-    if (R >= 0) any |= R < m.no_cells && m.material[R] == 0;
-    if (kind == 4 || !any)
+    float *Fo = F + ((int64_t)f * NG + g) * 5;
+    const int4 r = m.frec[f];
+    const int type = r.z & 15;
+    if (type == FF_NONE)
     {
 #pragma unroll
         for (int q = 0; q < 5; ++q) Fo[q] = 0.f;
@@ -574,35 +562,28 @@ __device__ __forceinline__ void mx_flux_one(const MV &m, const MxParams &p, int 
     }
     const float4 nf4 = m.fn[f];
     const float3 nr = f3(nf4);
-    const char2 sl = m.fslot[f];
-    // reconstructed face state of cell c (positivity fallback already applied by k_mx_grad): slot j of the
+    // reconstructed face state at entry 4 c + j (positivity fallback already applied by k_mx_grad): slot j of the
     // cell's float4 of each variable
-    const int64_t qs = 4 * n * ng;
-    auto state = [&](int32_t c, int side) {
-        const float *b = FV + ((int64_t)c * ng + g) * 4 + (side == 0 ? sl.x : sl.y);
+    const int64_t qs = 4 * (int64_t)m.nc * NG;
+    auto state = [&](int32_t k) {
+        const float *b = FV + ((int64_t)(k >> 2) * NG + g) * 4 + (k & 3);
         return F5{b[0], b[qs], b[2 * qs], b[3 * qs], b[4 * qs]};
     };
     F5 Ls, Rs;
-    if (cnt == 2 && kind == 0)
+    if (type == FF_INTERIOR)
     {
-        Ls = state(L, 0);
-        Rs = state(R, 1);
+        Ls = state(r.x);
+        Rs = state(r.y);
     }
     else
     {
         // the one fluid cell of a boundary / interface face (FluxRHS.cpp:58-66)
-        int32_t c = m.f2c_idx[p0];
-        int sgn = m.f2c_sgn[p0];
-        if (cnt == 2 && m.material[c] != 0)
-        {
-            c = m.f2c_idx[p0 + 1];
-            sgn = m.f2c_sgn[p0 + 1];
-        }
-        const F5 in = state(c, sgn > 0 ? 0 : 1);
-        const float sf = static_cast<float>(sgn);
+        const int kind = r.z >> 4;
+        const F5 in = state(r.x);
+        const float sf = type == FF_INSIDE_L ? 1.f : -1.f;
         F5 gh;
         if (!wall_ghost32(p, kind, f, s, gh)) gh = ghost32(kind, p.absorb[s] != 0, in, make_float3(sf * nr.x, sf * nr.y, sf * nr.z), p.fs[s]);
-        if (sgn > 0) { Ls = in; Rs = gh; }
+        if (type == FF_INSIDE_L) { Ls = in; Rs = gh; }
         else { Rs = in; Ls = gh; }
     }
     float Fl[5];
@@ -894,23 +875,24 @@ __global__ void k_mx_face_edges(MeshView m, int4 *fe)
 // write adjacent halves of the face's flux record, so every gather and store of the pair shares its
 // sectors.  The update keeps the group's species in one thread per cell and gathers each face's record
 // once for both.
-__global__ void __launch_bounds__(128) k_mx_grad(MV m, MxParams p, int s0, int ng, const float4 *__restrict__ W,
-                                                 float4 *__restrict__ FV)
+template <int NG>
+__global__ void __launch_bounds__(128) k_mx_grad(MV m, MxParams p, int s0, const float4 *__restrict__ W, float4 *__restrict__ FV)
 {
     pdl_begin();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t c = ng == 2 ? t >> 1 : t;
+    const int64_t c = t / NG;
     if (c >= m.nc) return;
-    mx_grad_one(m, p, s0, ng == 2 ? static_cast<int>(t & 1) : 0, ng, static_cast<int32_t>(c), W, FV);
+    mx_grad_one<NG>(m, p, s0, static_cast<int>(t % NG), static_cast<int32_t>(c), W, FV);
 }
 
-__global__ void __launch_bounds__(128) k_mx_flux(MV m, MxParams p, int s0, int ng, const float *__restrict__ FV, float *__restrict__ F)
+template <int NG>
+__global__ void __launch_bounds__(128) k_mx_flux(MV m, MxParams p, int s0, const float *__restrict__ FV, float *__restrict__ F)
 {
     pdl_begin();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t f = ng == 2 ? t >> 1 : t;
+    const int64_t f = t / NG;
     if (f >= m.nf) return;
-    mx_flux_one(m, p, s0, ng == 2 ? static_cast<int>(t & 1) : 0, ng, static_cast<int32_t>(f), FV, F);
+    mx_flux_one<NG>(m, p, s0, static_cast<int>(t % NG), static_cast<int32_t>(f), FV, F);
 }
 
 // gyr: the closing half-step gyration of the Strang splitting (mercury::gyrate, FP64 on the averaged
@@ -1118,10 +1100,10 @@ void mixed_setup(MhdState *st)
     t.K.alloc(16 * nc); t.recon.alloc(12 * nc); t.vol_inv.alloc(nc);
     if (st->src.on) st->g32.alloc(nf);
     if (st->src.ambi) st->d32.alloc(nf);
-    t.fn.alloc(nf); t.fdx.alloc(6 * nf); t.fslot.alloc(nf); t.fe.alloc(nf);
+    t.fn.alloc(nf); t.fe.alloc(nf);
     t.eth.alloc(ne); t.emode.alloc(ne); t.emn.alloc(nnz_e2f); t.esw.alloc(nnz_e2f);
     if (nc) k_mx_cells<<<grid_for(nc, 128), 128, 0, s>>>(m, t.K.p, t.recon.p, t.vol_inv.p);
-    if (nf) k_mx_faces<<<grid_for(nf, 256), 256, 0, s>>>(m, t.fn.p, t.fdx.p, t.fslot.p);
+    if (nf) k_mx_faces<<<grid_for(nf, 256), 256, 0, s>>>(m, t.fn.p);
     if (nf) k_mx_face_edges<<<grid_for(nf, 256), 256, 0, s>>>(m, t.fe.p);
     if (ne) k_mx_edges<<<grid_for(ne, 128), 128, 0, s>>>(m, t.eth.p, t.emode.p, t.emn.p, t.esw.p);
     MHD_LAUNCH_CHECK();
@@ -1232,13 +1214,13 @@ void mixed_stage(MhdState *st, const double *Us, const double *phis, double *Uo,
     {
         const int ng = std::min(st->group, st->nsp - s0);
         P.begin(KP_GRAD, s);
-        launch_pdl(k_mx_grad, grid_for(static_cast<int64_t>(m.nc) * ng, 128), 128, 0, s, m, p, s0, ng, W4,
+        launch_pdl(ng == 2 ? k_mx_grad<2> : k_mx_grad<1>, grid_for(static_cast<int64_t>(m.nc) * ng, 128), 128, 0, s, m, p, s0, W4,
                                                                                    reinterpret_cast<float4 *>(st->grad32.p));
         MHD_LAUNCH_CHECK();
         P.end(KP_GRAD, s);
         if (s0 == 0) emf_faces();
         P.begin(KP_FLUX, s);
-        launch_pdl(k_mx_flux, grid_for(static_cast<int64_t>(m.nf) * ng, 128), 128, 0, s, m, p, s0, ng, st->grad32.p, st->F32.p);
+        launch_pdl(ng == 2 ? k_mx_flux<2> : k_mx_flux<1>, grid_for(static_cast<int64_t>(m.nf) * ng, 128), 128, 0, s, m, p, s0, st->grad32.p, st->F32.p);
         MHD_LAUNCH_CHECK();
         P.end(KP_FLUX, s);
         if (s0 == 0)
