@@ -823,8 +823,9 @@ __global__ void __launch_bounds__(128, 4) k_a_edge(MeshView m, const double *__r
 
 // K2: face adjoint of k_face_candidate.  lEf_f = sum over the face's edges of w_ef lc_e t_e (fw: w_ef by f2e
 // entry), then E_f = -n x F back to u, B_tot, B_ind of the face's cells (atomic) and Phi_f; plus the edges'
-// upwind (efphi through efpos: the e2f entry of each f2e entry) and resistive (star2 sgn lres) terms.
-__global__ void __launch_bounds__(128) k_a_face_cand(MeshView m, const double *__restrict__ u, const double *__restrict__ Bt,
+// upwind (efphi through efpos: the e2f entry of each f2e entry) and resistive (star2 sgn lres) terms.  295k tetrahedra:
+// 34 us with 40 warps an SM, 37 with 28.
+__global__ void __launch_bounds__(128, 10) k_a_face_cand(MeshView m, const double *__restrict__ u, const double *__restrict__ Bt,
                                                       const double *__restrict__ Bi, const double *__restrict__ phi,
                                                       const double *__restrict__ phi_add, const double *__restrict__ lc,
                                                       const double *__restrict__ fw, const int32_t *__restrict__ efpos,
@@ -1013,8 +1014,9 @@ __device__ __forceinline__ void ghost_T(int kind, bool absorb, V3 n, const doubl
 // the reverse Rusanov flux at the face values FV that the forward stage left, the ghost state; writes the adjoint of each
 // cell's face state into its slot lface[((s*2 + side)*5 + q)*nf + f] (side 0: the cell with c2f sign +1).  Species 0
 // also adds the cell-fit transpose n_f . (y_L + y_R) to lphi.
-// 295k tetrahedra, two species: 76 us, 94 from the gradients.
-__global__ void __launch_bounds__(128) k_a_flux(MeshView m, FluidParams p, const double *__restrict__ FV, const double *__restrict__ lrV,
+// Bound by the latency of its gathers: 72 registers with some spills against 128 without.  295k tetrahedra, two
+// species: 60 us (16 warps an SM: 76, 20: 71), 94 from the gradients.
+__global__ void __launch_bounds__(128, 7) k_a_flux(MeshView m, FluidParams p, const double *__restrict__ FV, const double *__restrict__ lrV,
                                                  double *__restrict__ lface, double *__restrict__ lfs, const double *__restrict__ y,
                                                  double *__restrict__ lphi)
 {
@@ -1093,8 +1095,9 @@ __device__ __forceinline__ double ghost_q(int kind, bool absorb, int q, const do
 // stage ran with zero gradients (every face state the cell's).
 // The limiter term that sets psi is the forward pass's: the quotient at the largest or the most negative dl, the first
 // face that has it, the earlier one where the two quotients tie.
-// 295k tetrahedra, two species: 170 us, 228 as one thread per (cell, species) (168 registers, spills).
-__global__ void __launch_bounds__(160, 4) k_a_grad(MeshView m, FluidParams p, int second, const double *__restrict__ W,
+// Bound by latency and the FP64 divides: 72 registers, 25 warps an SM.  295k tetrahedra, two species: 153 us (20 warps:
+// 170, 30: 159), 228 as one thread per (cell, species) (168 registers, spills).
+__global__ void __launch_bounds__(160, 5) k_a_grad(MeshView m, FluidParams p, int second, const double *__restrict__ W,
                                                    const double *__restrict__ lface, double *__restrict__ lW, double *__restrict__ slot,
                                                    double *__restrict__ lfs)
 {
