@@ -112,7 +112,7 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
         g, e2f, f2e, ec = group, c["e2f"], c["f2e"], c["ec"]
         # limited_gradients: primitives (32 B per cell and species), stencil operator K (64 B) and neighbour ids (16 B),
         #   validity, face values out (80 B per cell and species)
-        # face_flux: face values of both sides, flux records out, per-face normal, slots, L/R, kind, f2c row
+        # face_flux: face values of both sides, flux records out, per-face normal and record (entries, kind)
         # update: flux records, face ids and signs, U in and out, U of the averaged stage (stage 2: the mean over
         #   the two launches is 20 B per species), 1/V, material
         # edge_emf: tangent + length, mode, row pointers, E out; per (edge, face) id and the 24-byte plane table;
@@ -122,7 +122,7 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
             "prepare": 40 * nsp * nc + 20 * nsp * nc + 16 * nc + 48 * nc + 8 * nf + 16 * nc + 48 * nc + nc,
             "cfl": 20 * nsp * nc + 16 * nc + 16 * nc + 16 * nf + 4 * nc + nc,
             "limited_gradients": 32 * g * nc + 64 * nc + 16 * nc + nc + 80 * g * nc,
-            "face_flux": 80 * g * nc + 20 * g * nf + 35 * nf + nc,
+            "face_flux": 80 * g * nc + 20 * g * nf + 32 * nf,
             "update": 20 * g * nf + 20 * nc + 40 * g * nc + 40 * g * nc + 20 * g * nc + 4 * nc + nc,
             "face_candidate": 48 * nc + 16 * nf + 16 * nf + 8 * nf + 12 * nf,
             "edge_emf": 29 * ne + 28 * e2f + 4 * ec + 16 * nf + 16 * nc,
@@ -134,21 +134,23 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
         return (10 * nsp * nc + nf * 5 + 3 * nc + 9 * nc) * p + csr_c2f + nc
     if k == "limited_gradients":
         g = group
-        return (20 * g * nc + 6 * nc + 3 * c["c2f"] + 3 * nc + 3 * nf) * p + c["c2f"] * 8 + csr_c2f + 2 * nc
+        # primitives in, face values out (one per variable and c2f slot), the stencil tables, neighbour ids, signs
+        return (5 * g * nc + 5 * g * c["c2f"] + 6 * nc + 6 * c["c2f"]) * p + c["c2f"] * 5 + nc
     if k == "face_flux":
         g = group
-        return (20 * g * nc + 3 * nc + 7 * nf + 5 * g * nf) * p + c["f2c"] * 5 + nf * 4 + 2 * nf * 4 + nf + nc
+        # face values of both sides, fluxes out, the face's normal and record
+        return (5 * g * c["c2f"] + 4 * nf + 5 * g * nf) * p + 16 * nf
     if k == "update":
         g = group
         return (5 * g * nf + 12.5 * g * nc + nc) * p + c["c2f"] * 5 + nc * 4 + nc   # stage 1 / 2 averaged (U0 read in stage 2)
     # face_candidate also writes phi_ind / |A| per face for the edge pass; edge_emf reads the per-(edge, slot)
     # face geometry (m, n, sigma, w: 8 values per e2f entry) instead of the faces' centres and areas
     if k == "face_candidate":
-        return (9 * nc + 4 * nf + 2 * nf + 3 * nf + nf) * p + c["f2c"] * 5 + nf * 4 + 2 * nf * 4
+        return (9 * nc + 4 * nf + 2 * nf + 3 * nf + nf) * p + 2 * nf * 4
     if k == "edge_emf":
         return (8 * c["e2f"] + 4 * ne + 3 * nf + nf + 3 * nc + ne) * p + c["e2f"] * 4 + ne * 8 + c["ec"] * 4 + nc + ne
     if k == "ct":
-        return (ne + 2.5 * nf) * p + c["f2e"] * 5 + nf * 4 + c["f2c"] * 4 + nf * 4
+        return (ne + 2.5 * nf) * p + c["f2e"] * 5
     if k == "cfl":
         return (5 * nsp * nc + 3 * nc + 4 * nf + nc) * p + csr_c2f + nc
     return 0.0

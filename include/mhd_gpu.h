@@ -277,7 +277,7 @@ int mhd_gpu_induction_set_ideal(MhdInduction *ind, const double *u_cell, const i
 int mhd_gpu_induction_ideal_linear(MhdInduction *ind, const double *phi, double *out);
 /* Per-kernel-class device time of the solve (CUDA events on the mesh stream while enabled; classes:
  * face_d1, cell_field, hall_emf, edge_gather, gram_schmidt, krylov_scalar, krylov_vector, ilu, ideal_emf; a profiled solve
- * launches its kernels one by one instead of replaying the restart-cycle graph), read as
+ * launches its kernels one by one instead of replaying the restart-cycle graphs), read as
  * in mhd_gpu_state_profile_read; and the number of kernels the handle has launched. */
 int mhd_gpu_induction_profile(MhdInduction *ind, int32_t enable);
 int mhd_gpu_induction_profile_read(MhdInduction *ind, int32_t max_kernels, char *names, double *ms_total, int64_t *count,

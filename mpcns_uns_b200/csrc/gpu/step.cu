@@ -344,6 +344,11 @@ void prepare_cfl(MhdState *st, const double *Us, const double *phis, bool cfl, d
         // grad p_e and the nodal p_e below need the primitives before the gyration
         launch_prepare(st, Us, phis, cfl, dt_max, turned && !st->src.ambi);
         ++st->launches;
+        if (P.on && st->src.on && !st->mixed) // J in the prepare class; without the profiler the stage launches it
+        {
+            launch_cell_current(m, st->bind.p, st->J.p, s);
+            ++st->launches;
+        }
         if (st->src.ambi && !st->mixed) // grad p_e (Solver.cpp:124) and the nodal p_e of the ambipolar EMF
         {
             launch_dpe(m, st->W.p, st->dpe.p, s);
@@ -376,11 +381,9 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
     cudaStream_t se = fork.emf;
     // the EMF chain in two halves, enqueued between the fluid's passes so that neither chain waits for the host
     auto emf_faces = [&] {
-        if (st->src.on && m.nc) // J of the induced field (Solver.cpp:123)
+        if (st->src.on && m.nc && !P.on) // J of the induced field (Solver.cpp:123)
         {
-            P.begin(KP_PREPARE, se);
             launch_cell_current(m, st->bind.p, st->J.p, se);
-            P.end(KP_PREPARE, se);
             ++st->launches;
         }
         fork.faces_done();
