@@ -1092,7 +1092,7 @@ __device__ __forceinline__ double ghost_q(int kind, bool absorb, int q, const do
 // blockDim = (32, 5) as k_limited_slots: warp q handles variable q of 32 cells with the stencil staged in shared memory.
 // The density and pressure warps tell the others which face states extrapolate; a wall or inflow ghost mixes the
 // variables, so the boundary slots' adjoints meet in shared memory and warp 0 takes them back.  second = 0: the forward
-// stage ran with zero gradients (every face state the cell's).
+// stage ran with zero gradients, every face state is the cell's, so the face adjoints add to it and no stencil sees any.
 // The limiter term that sets psi is the forward pass's: the quotient at the largest or the most negative dl, the first
 // face that has it, the earlier one where the two quotients tie.
 // Bound by latency and the FP64 divides: 72 registers, 25 warps an SM.  295k tetrahedra, two species: 153 us (20 warps:
@@ -1259,7 +1259,7 @@ __global__ void __launch_bounds__(160, 5) k_a_grad(MeshView m, FluidParams p, in
         double lG0 = 0, lG1 = 0, lG2 = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if ((pos[0][j] & pos[1][j]) >> lane & 1u)
+            if (second && (pos[0][j] & pos[1][j]) >> lane & 1u)
             {
                 lG0 += lf[j] * dx[3 * j][lane];
                 lG1 += lf[j] * dx[3 * j + 1][lane];
