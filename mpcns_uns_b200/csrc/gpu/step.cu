@@ -443,8 +443,13 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
         {
             if (st->prm.second_order) launch_limited_gradients(m, gp, Wg, Gg, s);
             else MHD_CUDA(cudaMemsetAsync(st->grad.p, 0, (size_t)15 * ng * nc * sizeof(double), s));
-            if (log && st->fv.n && st->floor_flags) launch_face_values(m, gp, Wg, false, nullptr, st->fv.p, s);
+            if (log && st->fv.n && st->floor_flags)
+            {
+                launch_face_values(m, gp, Wg, false, nullptr, st->fv.p, s);
+                st->launches += m.nc ? 1 : 0;
+            }
         }
+        st->launches += m.nc && (faces || st->prm.second_order) ? 1 : 0;
         P.end(KP_GRAD, s);
         if (s0 == 0) emf_faces();
         P.begin(KP_FLUX, s);
@@ -465,7 +470,7 @@ void stage(MhdState *st, const double *Us, const double *phis, double *Uo, doubl
             MHD_LAUNCH_CHECK();
             P.end(KP_UPDATE, s);
         }
-        st->launches += (st->prm.second_order && m.nc ? 1 : 0) + (m.nf ? 1 : 0) + (m.nc ? 1 : 0);
+        st->launches += (m.nf ? 1 : 0) + (m.nc ? 1 : 0);
     }
     if (gyrate_close) // the closing half-step gyration of Uo with this stage's Btot, beside the end of the EMF chain
     {
