@@ -28,6 +28,7 @@
 #include <array>
 #include <utility>
 
+#include "capture.cuh"
 #include "induction_op.cuh"
 
 namespace mhd
@@ -664,30 +665,23 @@ void build_cycle_graphs(MhdInduction *I)
     I->cycle_tried[md] = true;
     cudaStream_t s = I->mesh->stream;
     std::vector<MhdInduction::Chunk> chunks;
-    bool ok = true;
-    for (int j0 = 0; j0 < mr && ok; j0 += kCycleChunk)
+    for (int j0 = 0; j0 < mr; j0 += kCycleChunk)
     {
-        ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-        if (!ok) break;
         const int64_t l0 = I->launches;
         I->capturing = true;
-        enqueue_cycle(I, j0, std::min(mr, j0 + kCycleChunk));
-        I->capturing = false;
-        cudaGraph_t graph = nullptr;
         MhdInduction::Chunk c;
-        ok = cudaStreamEndCapture(s, &graph) == cudaSuccess && graph;
+        c.exec = capture_graph(s, [&] { enqueue_cycle(I, j0, std::min(mr, j0 + kCycleChunk)); });
+        I->capturing = false;
         c.kernels = I->launches - l0;
         I->launches = l0;
-        ok = ok && cudaGraphInstantiate(&c.exec, graph, 0) == cudaSuccess;
-        if (graph) cudaGraphDestroy(graph);
-        if (ok) chunks.push_back(c);
+        if (!c.exec)
+        {
+            for (auto &k : chunks) cudaGraphExecDestroy(k.exec);
+            return;
+        }
+        chunks.push_back(c);
     }
-    if (ok) I->cycle[md] = std::move(chunks);
-    else
-    {
-        cudaGetLastError();
-        for (auto &c : chunks) cudaGraphExecDestroy(c.exec);
-    }
+    I->cycle[md] = std::move(chunks);
 }
 
 // The cycle's steps up to limit: chunk k is launched when chunk k - 2 has finished without meeting the tolerance, so that
