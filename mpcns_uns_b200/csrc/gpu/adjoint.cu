@@ -580,6 +580,7 @@ __device__ __forceinline__ V3 recon_T(const MeshView &m, int32_t c, V3 lb)
 {
     const int64_t n = m.nc;
     const double *I = m.cinv + c;
+    if (cell_fit_skipped(m, c)) return mk(0, 0, 0);
     return mk(I[0] * lb.x + I[3 * n] * lb.y + I[6 * n] * lb.z, I[n] * lb.x + I[4 * n] * lb.y + I[7 * n] * lb.z,
               I[2 * n] * lb.x + I[5 * n] * lb.y + I[8 * n] * lb.z);
 }

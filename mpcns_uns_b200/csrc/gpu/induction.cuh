@@ -5,6 +5,14 @@
 
 namespace mhd
 {
+// A cell without a fit (a singular normal matrix) has a zero field, whatever its fluxes: the diagonal of an inverse is
+// positive, so three zeros mark it.
+__device__ __forceinline__ bool cell_fit_skipped(const MeshView &m, int32_t c)
+{
+    const int64_t n = m.nc;
+    return m.cinv[c] == 0 && m.cinv[4 * n + c] == 0 && m.cinv[8 * n + c] == 0;
+}
+
 // uns::reconstruct_cell_vector (src/uns/geometry/Reconstruct.cpp:8-46): area-weighted least squares
 // b . n_f = flux_f / A_f.  The normal matrix depends on the metric alone: its inverse comes from the mesh
 // (MeshView::cinv), and the right-hand side sum (s n)(s flux) is formed as sum n flux (the sign squares away exactly).
@@ -28,8 +36,9 @@ __device__ __forceinline__ V3 cell_vector(const MeshView &m, const double *__res
         for (int32_t k = m.c2f_ptr[c]; k < m.c2f_ptr[c + 1]; ++k) add(m.c2f_idx[k]);
     const int64_t n = m.nc;
     const double *I = m.cinv + c;
-    return mk(I[0] * r0 + I[n] * r1 + I[2 * n] * r2, I[3 * n] * r0 + I[4 * n] * r1 + I[5 * n] * r2,
-              I[6 * n] * r0 + I[7 * n] * r1 + I[8 * n] * r2);
+    const V3 b = mk(I[0] * r0 + I[n] * r1 + I[2 * n] * r2, I[3 * n] * r0 + I[4 * n] * r1 + I[5 * n] * r2,
+                    I[6 * n] * r0 + I[7 * n] * r1 + I[8 * n] * r2);
+    return cell_fit_skipped(m, c) ? mk(0, 0, 0) : b;
 }
 
 // (d1^T star2 phi)_e: the resistive current flux of ImplicitInduction::apply_F (ImplicitInduction.cpp:133-137)
