@@ -26,7 +26,10 @@ void set_last_error(const std::string &msg);
     do {                                                                                                       \
         cudaError_t e_ = (call);                                                                               \
         if (e_ != cudaSuccess)                                                                                 \
+        {                                                                                                      \
+            cudaGetLastError(); /* reported here: not again by the next call's launch check */                 \
             throw ::mhd::ApiError(MHD_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_));              \
+        }                                                                                                      \
     } while (0)
 #define MHD_REQUIRE(cond, msg)                                                                                 \
     do {                                                                                                       \
