@@ -1903,6 +1903,7 @@ int mhd_gpu_fn_create(MhdState *st, const MhdFnParams *p, const double *eta, con
         copy_d(fn->X0U.p, st->U0.p, 5 * fn->nsp * nc, s);
         copy_d(fn->X0P.p, st->phi0.p, nf, s);
         st->mres.alloc(ne);
+        st->fv.alloc(20 * nc * st->group); // the tape records face values: a state that was created without them gets them here
         fn->active.alloc(nf);
         fn->rslot.alloc(4 * nc);
         // f2e entries: as many as the e2f entries

@@ -20,6 +20,10 @@ struct ApiError : std::runtime_error
     int code;
     ApiError(int c, const std::string &m) : std::runtime_error(m), code(c) {}
 };
+struct OutOfMemory : ApiError // of the device
+{
+    using ApiError::ApiError;
+};
 void set_last_error(const std::string &msg);
 
 #define MHD_CUDA(call)                                                                                         \
@@ -88,7 +92,13 @@ template <class T> struct DBuf
         if (count)
         {
             g_alloc_calls.fetch_add(1, std::memory_order_relaxed);
-            MHD_CUDA(cudaMalloc(&p, count * sizeof(T)));
+            const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+            if (e == cudaErrorMemoryAllocation)
+            {
+                cudaGetLastError();
+                throw OutOfMemory(MHD_ECUDA, "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes: out of memory");
+            }
+            MHD_CUDA(e);
         }
         n = count;
     }

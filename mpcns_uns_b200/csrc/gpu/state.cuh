@@ -43,7 +43,7 @@ struct MhdState
     mhd::FluidParams fp{};
     int nsp = 0, group = 0;
     bool mixed = false;
-    mhd::DBuf<double> fv; // FP64 state on a mesh of one cell kind: face values (launch_face_values); others keep grad
+    mhd::DBuf<double> fv; // FP64 state on a mesh of one cell kind, if memory allows: face values (launch_face_values); others keep grad
     mhd::DBuf<double> U0, U1, W, grad, F, phi0, phi1, phi_add, badd, bind, btot, up, Ef, E, mass, stage;
     mhd::SrcParams src;     // two-ion J x B force and gyration (off unless params.lorentz)
     mhd::DBuf<double> J;    // cell current of the induced field (3 per cell) when the J x B force is on

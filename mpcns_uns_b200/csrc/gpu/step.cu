@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 
 #include "induction.cuh"
 #include "kernels.cuh"
@@ -548,110 +549,125 @@ int mhd_gpu_state_set_wall_ghosts(MhdState *st, int32_t n_wall, const int32_t *f
     });
 }
 
+// faces: an FP64 state on a mesh of one cell kind holds face values (launch_face_values), else gradients
+static MhdState *state_create(MhdMesh *mesh, const MhdStepParams *p, bool faces)
+{
+    MHD_REQUIRE(p->n_species >= 1 && p->n_species <= kMaxSpecies, "n_species must be 1..16");
+    MHD_REQUIRE(p->gamma > 1.0, "gamma must exceed 1");
+    for (int s = 0; s < p->n_species; ++s) MHD_REQUIRE(p->mass[s] > 0, "species masses must be positive");
+    MHD_REQUIRE(!p->lorentz || p->n_species == 2, "the J x B force and the gyration are those of the two-ion model (n_species == 2)");
+    MHD_REQUIRE(!(p->ambipolar || p->chemistry) || p->n_species == 2,
+                "the ambipolar and chemistry terms are those of the two-ion model (n_species == 2)");
+    MHD_REQUIRE(!p->ambipolar || mesh->v.e_nodes, "the ambipolar EMF needs the mesh's edge_nodes");
+    std::unique_ptr<MhdState> owner(new MhdState);
+    MhdState *st = owner.get();
+    st->mesh = mesh;
+    st->hold.take(mesh);
+    st->prm = *p;
+    st->nsp = p->n_species;
+    st->group = std::min(kGroup, st->nsp);
+    FluidParams &fp = st->fp;
+    fp.nsp = st->nsp;
+    fp.limit = 1;
+    fp.gamma = p->gamma;
+    fp.rel_limit = p->rel_limit;
+    fp.rho_floor = p->rho_floor;
+    fp.p_floor = p->p_floor;
+    for (int s = 0; s < st->nsp; ++s)
+    {
+        fp.fs[s] = Prim5{p->fs[s].rho, p->fs[s].u, p->fs[s].v, p->fs[s].w, p->fs[s].p};
+        fp.absorb[s] = p->absorb[s];
+    }
+    const MeshView &m = mesh->v;
+    const size_t nc = m.nc, nf = m.nf, ne = m.ne;
+    st->U0.alloc(5 * nc * st->nsp);
+    st->U1.alloc(5 * nc * st->nsp);
+    st->W.alloc(5 * nc * st->nsp);
+    if (p->precision != MHD_PREC_MIXED)
+    {
+        if (m.faces_per_cell && faces) st->fv.alloc(5 * (size_t)m.faces_per_cell * nc * st->group);
+        else st->grad.alloc(15 * nc * st->group);
+        st->F.alloc(5 * nf * st->group);
+    }
+    st->phi0.alloc(nf);
+    st->phi1.alloc(nf);
+    st->phi_add.alloc(nf);
+    st->badd.alloc(3 * nc);
+    st->bind.alloc(3 * nc);
+    st->btot.alloc(3 * nc);
+    st->up.alloc(3 * nc);
+    st->Ef.alloc(3 * nf);
+    st->E.alloc(ne);
+    st->stage.alloc(std::max<size_t>(5 * nc, 3 * nc));
+    st->scal.alloc(4);
+    st->dt_bits.alloc(1);
+    st->flag.alloc(1);
+    st->cfl_count.alloc(1);
+    st->mass.upload(p->mass, st->nsp);
+    st->src = src_params(*p);
+    if (st->src.on) st->J.alloc(3 * nc);
+    if (st->src.ambi)
+    {
+        if (p->precision != MHD_PREC_MIXED) st->dpe.alloc(3 * nc); // the mixed update gathers grad p_e itself
+        st->pn.alloc(m.nn ? (size_t)m.nn : 1);
+        st->pok.alloc(m.nn ? (size_t)m.nn : 1);
+    }
+    MHD_CUDA(cudaMallocHost(&st->pinned, 8 * sizeof(double)));
+    MHD_REQUIRE(p->precision == MHD_PREC_FP64 || p->precision == MHD_PREC_MIXED, "unknown precision");
+    st->mixed = p->precision == MHD_PREC_MIXED;
+    if (st->mixed)
+    {
+        MHD_REQUIRE(!m.nc || (m.faces_per_cell == 4 && m.tri_faces), "mixed precision needs a tetrahedral mesh");
+        MHD_REQUIRE(m.max_valence <= 8 && m.max_edge_cells <= 8, "mixed precision needs edge valence <= 8");
+        mixed_setup(st);
+    }
+    else
+    {
+        // the FP64 UCT's face geometry per (edge, slot) (512 bytes per edge), where the memory allows it:
+        // without it the edge pass forms the same values inline
+        const size_t n_geo = size_t(64) * ne;
+        size_t free_b = 0, total_b = 0;
+        MHD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (n_geo && m.max_edge_cells <= 8 && m.max_valence <= 8 && free_b > n_geo * sizeof(double) + (size_t(8) << 30))
+        {
+            st->efgeo.alloc(n_geo);
+            st->pa.alloc(nf);
+            build_edge_face_geo(m, st->efgeo.p, mesh->stream);
+        }
+    }
+    cudaStream_t s = mesh->stream;
+    if (nc) MHD_CUDA(cudaMemsetAsync(st->U0.p, 0, 5 * nc * st->nsp * sizeof(double), s));
+    if (nf)
+    {
+        MHD_CUDA(cudaMemsetAsync(st->phi0.p, 0, nf * sizeof(double), s));
+        MHD_CUDA(cudaMemsetAsync(st->phi_add.p, 0, nf * sizeof(double), s));
+    }
+    if (nc) MHD_CUDA(cudaMemsetAsync(st->badd.p, 0, 3 * nc * sizeof(double), s));
+    MHD_CUDA(cudaMemsetAsync(st->flag.p, 0, sizeof(int), s));
+    MHD_CUDA(cudaMemsetAsync(st->cfl_count.p, 0, sizeof(unsigned), s));
+    const double inf = HUGE_VAL;
+    MHD_CUDA(cudaMemcpyAsync(st->dt_bits.p, &inf, sizeof(inf), cudaMemcpyHostToDevice, s));
+    MHD_CUDA(cudaStreamSynchronize(s));
+    return owner.release();
+}
+
+// Face values take 20 doubles per tetrahedron and species, 30 per hexahedron; gradients 15.  Where the device's memory holds
+// a state only with the smaller ones, the steps go through them, with the same results (two species, a stage's passes to the
+// flux: 1.77M tetrahedra 357 + 198 us from face values, 309 + 507 from gradients; 307k hexahedra 118 + 59 and 95 + 136).
 int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *p, MhdState **out)
 {
-    MhdState *st = nullptr;
-    int rc = guarded([&] {
+    return guarded([&] {
         MHD_REQUIRE(mesh && p && out, "null argument");
-        MHD_REQUIRE(p->n_species >= 1 && p->n_species <= kMaxSpecies, "n_species must be 1..16");
-        MHD_REQUIRE(p->gamma > 1.0, "gamma must exceed 1");
-        for (int s = 0; s < p->n_species; ++s) MHD_REQUIRE(p->mass[s] > 0, "species masses must be positive");
-        MHD_REQUIRE(!p->lorentz || p->n_species == 2, "the J x B force and the gyration are those of the two-ion model (n_species == 2)");
-        MHD_REQUIRE(!(p->ambipolar || p->chemistry) || p->n_species == 2,
-                    "the ambipolar and chemistry terms are those of the two-ion model (n_species == 2)");
-        MHD_REQUIRE(!p->ambipolar || mesh->v.e_nodes, "the ambipolar EMF needs the mesh's edge_nodes");
-        st = new MhdState;
-        st->mesh = mesh;
-        st->hold.take(mesh);
-        st->prm = *p;
-        st->nsp = p->n_species;
-        st->group = std::min(kGroup, st->nsp);
-        FluidParams &fp = st->fp;
-        fp.nsp = st->nsp;
-        fp.limit = 1;
-        fp.gamma = p->gamma;
-        fp.rel_limit = p->rel_limit;
-        fp.rho_floor = p->rho_floor;
-        fp.p_floor = p->p_floor;
-        for (int s = 0; s < st->nsp; ++s)
+        try
         {
-            fp.fs[s] = Prim5{p->fs[s].rho, p->fs[s].u, p->fs[s].v, p->fs[s].w, p->fs[s].p};
-            fp.absorb[s] = p->absorb[s];
+            *out = state_create(mesh, p, true);
         }
-        const MeshView &m = mesh->v;
-        const size_t nc = m.nc, nf = m.nf, ne = m.ne;
-        st->U0.alloc(5 * nc * st->nsp);
-        st->U1.alloc(5 * nc * st->nsp);
-        st->W.alloc(5 * nc * st->nsp);
-        if (p->precision != MHD_PREC_MIXED)
+        catch (const OutOfMemory &)
         {
-            if (m.faces_per_cell) st->fv.alloc(5 * (size_t)m.faces_per_cell * nc * st->group);
-            else st->grad.alloc(15 * nc * st->group);
-            st->F.alloc(5 * nf * st->group);
+            if (!mesh->v.faces_per_cell || p->precision == MHD_PREC_MIXED) throw;
+            *out = state_create(mesh, p, false);
         }
-        st->phi0.alloc(nf);
-        st->phi1.alloc(nf);
-        st->phi_add.alloc(nf);
-        st->badd.alloc(3 * nc);
-        st->bind.alloc(3 * nc);
-        st->btot.alloc(3 * nc);
-        st->up.alloc(3 * nc);
-        st->Ef.alloc(3 * nf);
-        st->E.alloc(ne);
-        st->stage.alloc(std::max<size_t>(5 * nc, 3 * nc));
-        st->scal.alloc(4);
-        st->dt_bits.alloc(1);
-        st->flag.alloc(1);
-        st->cfl_count.alloc(1);
-        st->mass.upload(p->mass, st->nsp);
-        st->src = src_params(*p);
-        if (st->src.on) st->J.alloc(3 * nc);
-        if (st->src.ambi)
-        {
-            if (p->precision != MHD_PREC_MIXED) st->dpe.alloc(3 * nc); // the mixed update gathers grad p_e itself
-            st->pn.alloc(m.nn ? (size_t)m.nn : 1);
-            st->pok.alloc(m.nn ? (size_t)m.nn : 1);
-        }
-        MHD_CUDA(cudaMallocHost(&st->pinned, 8 * sizeof(double)));
-        MHD_REQUIRE(p->precision == MHD_PREC_FP64 || p->precision == MHD_PREC_MIXED, "unknown precision");
-        st->mixed = p->precision == MHD_PREC_MIXED;
-        if (st->mixed)
-        {
-            MHD_REQUIRE(!m.nc || (m.faces_per_cell == 4 && m.tri_faces), "mixed precision needs a tetrahedral mesh");
-            MHD_REQUIRE(m.max_valence <= 8 && m.max_edge_cells <= 8, "mixed precision needs edge valence <= 8");
-            mixed_setup(st);
-        }
-        else
-        {
-            // the FP64 UCT's face geometry per (edge, slot) (512 bytes per edge), where the memory allows it:
-            // without it the edge pass forms the same values inline
-            const size_t n_geo = size_t(64) * ne;
-            size_t free_b = 0, total_b = 0;
-            MHD_CUDA(cudaMemGetInfo(&free_b, &total_b));
-            if (n_geo && m.max_edge_cells <= 8 && m.max_valence <= 8 && free_b > n_geo * sizeof(double) + (size_t(8) << 30))
-            {
-                st->efgeo.alloc(n_geo);
-                st->pa.alloc(nf);
-                build_edge_face_geo(m, st->efgeo.p, mesh->stream);
-            }
-        }
-        cudaStream_t s = mesh->stream;
-        if (nc) MHD_CUDA(cudaMemsetAsync(st->U0.p, 0, 5 * nc * st->nsp * sizeof(double), s));
-        if (nf)
-        {
-            MHD_CUDA(cudaMemsetAsync(st->phi0.p, 0, nf * sizeof(double), s));
-            MHD_CUDA(cudaMemsetAsync(st->phi_add.p, 0, nf * sizeof(double), s));
-        }
-        if (nc) MHD_CUDA(cudaMemsetAsync(st->badd.p, 0, 3 * nc * sizeof(double), s));
-        MHD_CUDA(cudaMemsetAsync(st->flag.p, 0, sizeof(int), s));
-        MHD_CUDA(cudaMemsetAsync(st->cfl_count.p, 0, sizeof(unsigned), s));
-        const double inf = HUGE_VAL;
-        MHD_CUDA(cudaMemcpyAsync(st->dt_bits.p, &inf, sizeof(inf), cudaMemcpyHostToDevice, s));
-        MHD_CUDA(cudaStreamSynchronize(s));
-        *out = st;
     });
-    if (rc != MHD_OK) delete st;
-    return rc;
 }
 
 int mhd_gpu_state_destroy(MhdState *st)
