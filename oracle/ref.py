@@ -39,11 +39,15 @@ class StepParams(ctypes.Structure):
                 ("first_order", i32), ("ind_iterations", i32), ("ind", ctypes.c_void_p), ("ind_rel_res", dbl)]
 
 
+class NotBuilt(RuntimeError):
+    """The compiled reference is not on this machine (a test that asks for it is skipped)."""
+
+
 def lib():
     global _lib
     if _lib is None:
         if not available():
-            raise RuntimeError("reference checker not built: make -C oracle ref")
+            raise NotBuilt("reference checker not built: make -C oracle ref")
         L = ctypes.CDLL(SO)
         L.ref_last_error.restype = ctypes.c_char_p
         for name, args, res in [
