@@ -74,7 +74,6 @@ __device__ __forceinline__ double limiter_psi(double wc, double lo, double hi, d
 // q of 32 consecutive cells.  Each variable's fit and limiter are independent of the others (wall
 // ghosts only read the velocity), so the per-thread state is small, occupancy high, and the five
 // warps share the cell's geometry through L1.  The reference's arithmetic order is kept per variable.
-template <bool LOG>
 __global__ void __launch_bounds__(160) k_limited_gradients_v(MeshView m, FluidParams p, SField<const double> W, SField<double> G)
 {
     const int32_t c = blockIdx.x * 32 + threadIdx.x;
@@ -94,7 +93,6 @@ __global__ void __launch_bounds__(160) k_limited_gradients_v(MeshView m, FluidPa
     {
         const double wc = W(s, c, q);
         double lo = wc, hi = wc, r0 = 0, r1 = 0, r2 = 0;
-        int jlo = 7, jhi = 7, jpos = 7, jneg = 7; // switch log: the slots of the extremes
         for (int32_t k = k0; k < k1; ++k)
         {
             const int32_t nb = m.st_nb[k];
@@ -116,8 +114,6 @@ __global__ void __launch_bounds__(160) k_limited_gradients_v(MeshView m, FluidPa
             r0 += m.st_wd[3 * (int64_t)k] * dq;
             r1 += m.st_wd[3 * (int64_t)k + 1] * dq;
             r2 += m.st_wd[3 * (int64_t)k + 2] * dq;
-            if (LOG && wn < lo) jlo = k - k0;
-            if (LOG && hi < wn) jhi = k - k0;
             lo = dmin(lo, wn);
             hi = dmax(hi, wn);
         }
@@ -132,15 +128,10 @@ __global__ void __launch_bounds__(160) k_limited_gradients_v(MeshView m, FluidPa
             {
                 const V3 dx = ld3(m.face_center, m.c2f_idx[k]) - xc;
                 const double dl = g0 * dx.x + g1 * dx.y + g2 * dx.z;
-                if (LOG && dl > dpos) jpos = k - k0;
-                if (LOG && dl < dneg) jneg = k - k0;
                 if (dl > dpos) dpos = dl;
                 if (dl < dneg) dneg = dl;
             }
             psi = limiter_psi(wc, lo, hi, dpos, dneg, p.rel_limit > 0 && (q == 0 || q == 4) ? p.rel_limit : 0.0);
-            if (LOG)
-                sw_log(p.sw_lim, (s * 5 + q) * (int64_t)m.nc + c,
-                       limiter_code(psi, wc, lo, hi, dpos, dneg, jlo, jhi, jpos, jneg, p.rel_limit, p.rel_limit > 0 && (q == 0 || q == 4)));
         }
         const double ps = dmax(0.0, dmin(1.0, psi));
         G(s, c, 3 * q) = ps * g0;
@@ -531,11 +522,11 @@ __global__ void k_gather_rhs(MeshView m, int nsp, const double *__restrict__ F, 
 void launch_limited_gradients(const MeshView &m, const FluidParams &p, SField<const double> W, SField<double> G, cudaStream_t s)
 {
     if (!m.nc) return;
-    const bool log = p.sw_lim && p.limit;
-    if (m.faces_per_cell == 4) (log ? launch_slots<4, true, true, false> : launch_slots<4, false, true, false>)(m, p, W, G, nullptr, s);
-    else if (m.faces_per_cell == 6)
-        (log ? launch_slots<6, true, true, false> : launch_slots<6, false, true, false>)(m, p, W, G, nullptr, s);
-    else (log ? k_limited_gradients_v<true> : k_limited_gradients_v<false>)<<<grid_for(m.nc, 32), dim3(32, 5), 0, s>>>(m, p, W, G);
+    // the switch log is the differentiated run's, which needs tetrahedra
+    if (m.faces_per_cell == 4)
+        (p.sw_lim && p.limit ? launch_slots<4, true, true, false> : launch_slots<4, false, true, false>)(m, p, W, G, nullptr, s);
+    else if (m.faces_per_cell == 6) launch_slots<6, false, true, false>(m, p, W, G, nullptr, s);
+    else k_limited_gradients_v<<<grid_for(m.nc, 32), dim3(32, 5), 0, s>>>(m, p, W, G);
     MHD_LAUNCH_CHECK();
 }
 

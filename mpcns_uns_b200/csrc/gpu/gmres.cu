@@ -6,8 +6,8 @@
 // resistive current flux reaches an edge from its faces in ascending face order (e2f rows), the Hall
 // EMF from its cells in ascending cell order (ec rows, the reference's ce lists); the FP64 operator
 // is therefore reference-exact.  The Krylov part keeps H, g and the Givens rotations on the device;
-// the host reads one value per Arnoldi step (the early-exit test) and one per restart (the true
-// residual).  Its dot products are deterministic block reductions, whose rounding differs from the
+// the host reads the early-exit flag, from pinned memory, before it launches a further chunk of kCycleChunk
+// Arnoldi steps, and the true residual once per restart.  Its dot products are deterministic block reductions, whose rounding differs from the
 // reference's sequential sums, so GMRES iterates agree to the solver tolerance, not bit for bit.
 //
 // Fusions of the Arnoldi step (each keeps the reference's arithmetic per element):
@@ -23,8 +23,8 @@
 //     tail of w and V_{i-1} left in L2 is reused first;
 //   * every dot of the operator finishes in the kernel that produces it (the last block adds the block partials), those
 //     of Gram-Schmidt in k_cgs_tail, which also rotates the column, and
-//     a restart cycle runs as CUDA graphs of a few steps whose kernels test a device-side flag, so the host does not
-//     wait for the device within a restart.
+//     a restart cycle runs as CUDA graphs of kCycleChunk steps whose kernels test a device-side flag; the host waits for
+//     chunk k - 2 before it launches chunk k, so that the device has the next chunk queued while one runs.
 #include <array>
 #include <utility>
 

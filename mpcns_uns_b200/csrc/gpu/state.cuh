@@ -8,7 +8,8 @@
 
 namespace mhd
 {
-// Kernel classes of the step, timed with CUDA events on the handle's stream when profiling is on.
+// Kernel classes of the step, timed with CUDA events on the handle's stream when profiling is on.  "cfl" keeps its place in
+// the list that callers read, but the CFL step is part of the prepare pass and no launch has that class.
 enum StepKernel { KP_PREPARE = 0, KP_CFL, KP_GRAD, KP_FLUX, KP_UPDATE, KP_FACE_CAND, KP_EDGE_EMF, KP_CT, KP_GYRATE, KP_COUNT };
 static const char *const kStepKernelNames[KP_COUNT] = {"prepare", "cfl",            "limited_gradients", "face_flux", "update",
                                                         "face_candidate", "edge_emf", "ct",                "gyrate"};

@@ -3,12 +3,13 @@
 // reference operation order, no multiply-add contraction).
 //
 // One stage on (Us, Phi_s) -> (Uo, Phi_o):
-//   k_prepare      per cell: primitives of every species, B_ind = cell fit of Phi_s, B_tot, u+
-//   [k_cell_current] J of B_ind when the two-ion J x B force is on
-//   [k_cfl_*]      stage 1, CFL mode: per-cell step, device-wide minimum (no host round trip)
-//   per species group: k_limited_gradients, k_face_flux, k_update (gather [+ J x B] + U += dt rhs + floors)
-//   k_face_candidate, k_edge_emf_assign (begin + UCT + boundary edge values)
-//   k_ct           Phi_o = Phi_s - dt d1 E on the active faces
+//   k_prepare      per cell: primitives of every species, B_ind = cell fit of Phi_s, B_tot, u+; in stage 1 and CFL mode
+//                  also the cell's step and its device-wide minimum (no host round trip)
+//   the mesh's stream, per species group: k_limited_slots (limited face values), k_face_flux_fv, k_update (gather
+//                  [+ J x B] + U += dt rhs + floors); general polyhedra: k_limited_gradients_v, k_face_flux
+//   its side stream: [k_cell_current] J of B_ind when the two-ion J x B force is on, k_face_candidate,
+//                  k_edge_emf_assign (begin + UCT + boundary edge values),
+//                  k_ct  Phi_o = Phi_s - dt d1 E on the active faces
 // Stage 2 writes the SSP-RK2 averages U = (U0 + U2)/2, Phi = (Phi0 + Phi2)/2 in place.  With the
 // gyration on, half-step exact gyrations (k_gyrate) wrap the two stages (Strang splitting).
 #include <math_constants.h>
