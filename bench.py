@@ -101,7 +101,8 @@ def algorithmic_bytes(k, c, nsp, group, precision="fp64", sources=False):
         extra = {"face_candidate": 16 * nf, "update": 16 * nf + 16 * nc,
                  "gyrate": gyr + 16 * nc + 20 * nsp * nc + 16 * nc}
     else:
-        extra = {"prepare": 64 * nc + c["c2f"] * 5 + 36 * nf, "update": (2 + 3 + 3) * 8 * nc,
+        # the cell current (timed in the prepare class): the field in, J out, 1/V; face ids and signs, areas and cells
+        extra = {"prepare": 56 * nc + c["c2f"] * 5 + 32 * nf, "update": (2 + 3 + 3) * 8 * nc,
                  "gyrate": gyr + 24 * nc + (40 * nsp * nc + 24 * nc) / 2}
     return base + extra.get(k, 0.0)
 
@@ -110,6 +111,9 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
     nc, nf, ne = c["nc"], c["nf"], c["ne"]
     if precision == "mixed":
         g, e2f, f2e, ec = group, c["e2f"], c["f2e"], c["ec"]
+        # prepare: U in, primitives (32 B) and u+ out, face ids, the fit's operator (48 B), Phi, the background field,
+        #   both cell fields out, material; the CFL step (one of the two launches) the faces' normals and 1/V
+        # cfl: what the step size reads; it is formed in prepare, so no launch has this class and its time reads 0
         # limited_gradients: primitives (32 B per cell and species), stencil operator K (64 B) and neighbour ids (16 B),
         #   validity, face values out (80 B per cell and species)
         # face_flux: face values of both sides, flux records out, per-face normal and record (entries, kind)
@@ -119,7 +123,8 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
         #   per (edge, cell) id; the faces' 16-byte EMF records and the cells' velocities
         # ct: the packed face-edge record, Phi in, Phi out, the averaged Phi (mean 4 B), E
         return {
-            "prepare": 40 * nsp * nc + 20 * nsp * nc + 16 * nc + 48 * nc + 8 * nf + 16 * nc + 48 * nc + nc,
+            "prepare": 40 * nsp * nc + 32 * nsp * nc + 16 * nc + 16 * nc + 48 * nc + 8 * nf + 16 * nc + 32 * nc + nc
+                       + (16 * nf + 4 * nc) / 2,
             "cfl": 20 * nsp * nc + 16 * nc + 16 * nc + 16 * nf + 4 * nc + nc,
             "limited_gradients": 32 * g * nc + 64 * nc + 16 * nc + nc + 80 * g * nc,
             "face_flux": 80 * g * nc + 20 * g * nf + 32 * nf,
@@ -129,9 +134,10 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
             "ct": 36 * nf + 4 * ne,
         }.get(k, 0.0)
     p = 8
-    csr_c2f = c["c2f"] * 5 + nc * 4          # idx + sgn + ptr
     if k == "prepare":
-        return (10 * nsp * nc + nf * 5 + 3 * nc + 9 * nc) * p + csr_c2f + nc
+        # U in, primitives out, Phi and the faces' normals, the background field, both cell fields and u+ out, the fit's
+        # inverse; the volumes for the CFL step (one of the two launches); face ids, material
+        return (10 * nsp * nc + 5 * nf + 3 * nc + 9 * nc + 9 * nc + nc / 2) * p + c["c2f"] * 4 + nc
     if k == "limited_gradients":
         g = group
         # primitives in, face values out (one per variable and c2f slot), the stencil tables, neighbour ids, signs
@@ -151,8 +157,8 @@ def _algorithmic_bytes(k, c, nsp, group, precision="fp64"):
         return (8 * c["e2f"] + 4 * ne + 3 * nf + nf + 3 * nc + ne) * p + c["e2f"] * 4 + ne * 8 + c["ec"] * 4 + nc + ne
     if k == "ct":
         return (ne + 2.5 * nf) * p + c["f2e"] * 5
-    if k == "cfl":
-        return (5 * nsp * nc + 3 * nc + 4 * nf + nc) * p + csr_c2f + nc
+    if k == "cfl":  # formed in prepare: no launch has this class
+        return (5 * nsp * nc + 3 * nc + 4 * nf + nc) * p + c["c2f"] * 5 + nc * 4 + nc
     return 0.0
 
 
