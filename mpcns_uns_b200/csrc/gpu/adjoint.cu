@@ -580,9 +580,9 @@ __device__ __forceinline__ V3 recon_T(const MeshView &m, int32_t c, V3 lb)
 {
     const int64_t n = m.nc;
     const double *I = m.cinv + c;
-    if (cell_fit_skipped(m, c)) return mk(0, 0, 0);
-    return mk(I[0] * lb.x + I[3 * n] * lb.y + I[6 * n] * lb.z, I[n] * lb.x + I[4 * n] * lb.y + I[7 * n] * lb.z,
-              I[2 * n] * lb.x + I[5 * n] * lb.y + I[8 * n] * lb.z);
+    const V3 y = mk(I[0] * lb.x + I[3 * n] * lb.y + I[6 * n] * lb.z, I[n] * lb.x + I[4 * n] * lb.y + I[7 * n] * lb.z,
+                    I[2 * n] * lb.x + I[5 * n] * lb.y + I[8 * n] * lb.z);
+    return cell_fit_skipped(m, c) ? mk(0, 0, 0) : y; // chosen last: the nine loads are not held up (k_a_cell 18.5 us, 30.4 with a branch)
 }
 
 // lphi_f += n_f . (y_L + y_R), n_f = A_f / |A_f| (faces with |A_f| > 0)
