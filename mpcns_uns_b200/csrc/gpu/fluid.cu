@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(128) k_face_flux(MeshView m, FluidParams p, SF
 }
 
 // The same face flux from the face values that k_limited_slots<..., FACE> left: one 16-byte and one 32-byte record
-// per face, then 5 values per side.  Species in neighbouring blocks, which read the same records.  62% of the DRAM peak
+// per face, then 5 values per side.  Species in neighbouring blocks, which read the same records.  64% of the DRAM peak
 // on 1.77M tetrahedra, two species: 208 us a launch (78 registers: 214) against 482 from the gradients.
 __global__ void __launch_bounds__(128, 7) k_face_flux_fv(MeshView m, FluidParams p, int64_t nnz, const double *__restrict__ FV,
                                                       double *__restrict__ F)
