@@ -367,6 +367,8 @@ typedef struct MhdStepParams {
 #define MHD_FIELD_PHIADD 2 /* static background face flux; uploading it also sets the background cell field */
 #define MHD_FIELD_BADD 3   /* background cell field (3 per cell), download only */
 
+/* An FP64 state on tetrahedra or hexahedra holds limited face values, or where the device's memory is too short for them the
+ * smaller gradients; the steps give the same bits. */
 int mhd_gpu_state_create(MhdMesh *mesh, const MhdStepParams *params, MhdState **out);
 int mhd_gpu_state_destroy(MhdState *state);
 /* Host transfers in the reference layout (AoS); `species` selects the fluid for MHD_FIELD_U. */
